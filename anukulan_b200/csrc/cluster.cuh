@@ -184,7 +184,7 @@ __device__ __forceinline__ void cluster_phase(const RowSlice<T>& a, const Cluste
   for (int32_t r = a.rb + t; r < a.re; r += kClusterThreads) {
     if (a.start[r - a.rb + 1] - a.start[r - a.rb] > kSerialRow) continue;
     const typename Epi::Pre pre = epi.prefetch(r, 0);
-    const T v = epi.finish(r, 0, serial_row_sum(a, xs, r), pre);
+    const T v = epi.finish(r, 0, serial_row_sum(a, xs, r), pre, epi.params(0));
 #pragma unroll
     for (int q = 0; q < C; ++q) st_cluster(copy + r, q, v);
   }
@@ -196,7 +196,7 @@ __device__ __forceinline__ void cluster_phase(const RowSlice<T>& a, const Cluste
     if (lane == 0) pre = epi.prefetch(r, 0);
     const T s = warp_row_sum(a, xs, r, lane);
     if (lane == 0) {
-      const T v = epi.finish(r, 0, s, pre);
+      const T v = epi.finish(r, 0, s, pre, epi.params(0));
 #pragma unroll
       for (int q = 0; q < C; ++q) st_cluster(copy + r, q, v);
     }
