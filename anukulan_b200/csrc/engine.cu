@@ -125,29 +125,44 @@ void DevCsr::set_tile(int32_t threads) {
   tile_threads = threads;
 }
 
-void DevCsr::prepare_cluster(const HostCsr& a, cudaStream_t s) {
-  if (cl_ready) return;
-  auto put_rows = [&](DevBuf<int32_t>& d, const std::vector<int32_t>& h) {
-    d.alloc(std::max<size_t>(h.size(), 1));
+void DevCsr::prepare_cluster(const HostCsr& a, bool stack, int ctas, int32_t seg_nnz,
+                             cudaStream_t s) {
+  Cluster& d = clusters[stack][ctas == 8];
+  if (d.ready) return;
+  SegmentSchedule sch;
+  if (stack) sch = segment_schedule(a, seg_nnz, seg_per_cta, kSegRows);
+  const ClusterSchedule c = cluster_schedule(a, ctas, kSerialRow, stack ? &sch : nullptr);
+  auto put = [&](auto& buf, const auto& h) {
+    buf.alloc(std::max<size_t>(h.size(), 1));
+    static_assert(sizeof(*buf.p) == sizeof(h[0]), "host and device schedule entries");
     if (!h.empty())
-      ANU_CUDA(cudaMemcpyAsync(d.p, h.data(), sizeof(int32_t) * h.size(), cudaMemcpyHostToDevice, s));
+      ANU_CUDA(cudaMemcpyAsync(buf.p, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice, s));
   };
-  for (int i = 0; i < 2; ++i) {
-    const ClusterSchedule c = cluster_schedule(a, i == 0 ? 16 : 8, kSerialRow);
-    put_rows(cl_bounds[i], c.bounds);
-    put_rows(cl_warp_start[i], c.warp_start);
-    put_rows(cl_warp_rows[i], c.warp_rows);
-    cl_max_rows[i] = c.max_part_rows;
-    cl_max_nnz[i] = c.max_part_nnz;
-    max_row = c.max_row;
-  }
+  put(d.bounds, c.bounds);
+  put(d.part_start, c.part_start);
+  put(d.row, c.row);
+  put(d.part, c.part);
+  put(d.entry, c.entry);
   ANU_CUDA(cudaStreamSynchronize(s));
-  cl_ready = true;
+  d.rows = {d.bounds.p, d.part_start.p, d.row.p, d.part.p, nullptr, d.entry.p,
+            c.max_rows, c.max_entries, c.max_parts, c.stride};
+  d.row_place = c.place;
+  d.max_row = c.max_row;
+  d.ready = true;
 }
 
-ClusterRows DevCsr::cluster_rows(int ctas) const {
-  const int i = ctas == 16 ? 0 : 1;
-  return {cl_bounds[i].p, cl_warp_start[i].p, cl_warp_rows[i].p, cl_max_rows[i], cl_max_nnz[i]};
+void DevCsr::place_cluster(const HostCsr& a, const Cluster& other, bool stack, int ctas,
+                           cudaStream_t s) {
+  Cluster& d = clusters[stack][ctas == 8];
+  if (d.rows.place != nullptr) return;
+  std::vector<int32_t> h(a.index.size());
+  for (size_t e = 0; e < h.size(); ++e) h[e] = other.row_place[a.index[e]];
+  d.place.alloc(std::max<size_t>(h.size(), 1));
+  if (!h.empty())
+    ANU_CUDA(cudaMemcpyAsync(d.place.p, h.data(), sizeof(int32_t) * h.size(),
+                             cudaMemcpyHostToDevice, s));
+  ANU_CUDA(cudaStreamSynchronize(s));
+  d.rows.place = d.place.p;
 }
 
 template <>
@@ -1195,23 +1210,45 @@ void run_polish(Problem& p, bool unit, const std::vector<const CaseData*>& paren
                                       states[which[w]].scales);
 }
 
-// The cluster size cluster_chunk_kernel takes a single LP on `p` with, 0
-// where it does not take it: options.cluster_chunks off, a packed batch's
-// LP, a row longer than kLongRow, or y and x_bar too large for one CTA's
-// shared memory.
+// How K cases on `p` run as cluster-resident chunks (cluster_chunk_kernel):
+// clusters of 16 CTAs (8 where the device takes no cluster of 16), all of them
+// resident at once. Not taken where a CTA's rows exceed its threads or its
+// slices its shared memory, where a single LP has a row longer than kLongRow (which more
+// than a warp sums), or where the clusters would have to take turns.
 template <class T>
-int cluster_shape(Problem& p, const anu_pdhg_options& o) {
-  if (!o.cluster_chunks || p.concurrent || p.m == 0 || p.n == 0) return 0;
-  p.dk.prepare_cluster(p.k, p.stream);
-  p.dkt.prepare_cluster(p.kt, p.stream);
-  if (p.dk.max_row > kLongRow || p.dkt.max_row > kLongRow) return 0;
-  if (p.cluster_ctas < 0)
-    p.cluster_ctas =
-        cluster_ctas_for<T>(ClusterLayout::of<T>(p.m, p.n, p.dkt.cluster_rows(16),
-                                                 p.dk.cluster_rows(16)).total,
-                            ClusterLayout::of<T>(p.m, p.n, p.dkt.cluster_rows(8),
-                                                 p.dk.cluster_rows(8)).total);
-  return p.cluster_ctas;
+ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
+  ClusterPlan none;
+  if (p.m == 0 || p.n == 0 || p.dk.nnz == 0) return none;
+  // Before any schedule is built: the shares are even at best.
+  if (std::max(p.m, p.n) > 16 * kClusterThreadsMax ||
+      2 * sizeof(ClusterNz<T>) * (p.dk.nnz / 16) + sizeof(T) * (p.m + p.n) > kClusterSmemMax)
+    return none;
+  const auto key = std::make_pair(K, max_len);
+  const auto known = p.cluster_plans.find(key);
+  if (known != p.cluster_plans.end()) return known->second;
+  ClusterPlan plan;
+  const bool stack = K > 1;
+  for (const int ctas : {16, 8}) {
+    p.dk.prepare_cluster(p.k, stack, ctas, p.seg_nnz, p.stream);
+    p.dkt.prepare_cluster(p.kt, stack, ctas, p.seg_nnz, p.stream);
+    const DevCsr::Cluster &ck = p.dk.cluster(stack, ctas), &ckt = p.dkt.cluster(stack, ctas);
+    if (!stack && std::max(ck.max_row, ckt.max_row) > kLongRow) break;
+    const int32_t rows = std::max(ck.rows.max_rows, ckt.rows.max_rows);
+    if (rows > kClusterThreadsMax) break;
+    // Threads for the rows, and as far as there is room for the sums apart
+    // beside them: a warp each for a single LP, a thread each for a stack.
+    const int32_t parts = std::max(ck.rows.max_parts, ckt.rows.max_parts);
+    const int32_t want = std::max(128, stack ? rows + parts : std::max(rows, 32 * parts));
+    const int threads = std::min((want + 31) / 32 * 32, kClusterThreadsMax);
+    const size_t smem = ClusterLayout::of<T>(ctas, ckt.rows, ck.rows, max_len).total;
+    if (cluster_capacity<T>(cluster_kernel<T>(stack), ctas, threads, smem) < K) continue;
+    p.dk.place_cluster(p.k, ckt, stack, ctas, p.stream);
+    p.dkt.place_cluster(p.kt, ck, stack, ctas, p.stream);
+    plan = {ctas, threads, max_len};
+    break;
+  }
+  p.cluster_plans[key] = plan;
+  return plan;
 }
 
 template <class T>
@@ -1569,9 +1606,19 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
   // the rest.
   const bool persistent = o.persistent_chunks != 0 && !slow && o.use_graphs &&
                           chunk_fits<T>(p.dkt, p.dk, K);
-  // A single LP small enough runs each chunk as one cluster-resident launch
-  // (cluster_chunk_kernel); so does a stack's last case once compacted.
-  int cluster_c = (K == 1 && !persistent && !slow) ? cluster_shape<T>(p, o) : 0;
+  // A small enough matrix runs its chunks as cluster-resident launches
+  // (cluster_chunk_kernel).
+  ClusterPlan cp;
+  // Written by the device only when a wait in a cluster gave up.
+  Pinned<int32_t> h_cluster_status(1);
+  h_cluster_status.p[0] = 0;
+  auto plan_clusters = [&]() {
+    cp = ClusterPlan{};
+    if (persistent || slow || !o.use_graphs) return;
+    const int longest = o.cluster_chunks ? kClusterMaxLen : kClusterLaunchLen;
+    cp = cluster_plan<T>(p, K, std::min(F, longest));
+  };
+  plan_clusters();
   DevBuf<uint32_t> sync_arrived;
   DevBuf<int32_t> sync_status;
   Pinned<int32_t> h_sync_status(persistent ? 1 : 0);
@@ -1584,6 +1631,8 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
   }
   // After a synchronisation of the stream: the chunks before it are done.
   auto chunks_done = [&]() {
+    if (*static_cast<volatile int32_t*>(h_cluster_status.p) != 0)
+      throw Error(ANU_ERR_DEVICE_WAIT, "cluster_chunk_kernel: a wait for a peer's entries gave up");
     if (!persistent) return;
     if (coop_lock.owns_lock()) coop_lock.unlock();
     if (h_sync_status.p[0] != 0)
@@ -1647,16 +1696,22 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
                                cudaMemcpyDeviceToHost, st));
       return;
     }
-    if (cluster_c > 0 && K == 1 && len <= kClusterMaxLen) {
-      PrimalEpi<T> pe{K, 0, base_flags, w.params.p, w.w_table.p, w.x.p, w.x.p, w.c.p, w.lo.p,
-                      w.hi.p, w.x_bar.p, w.anchor_x.p, w.dx.p, w.sum_x.p};
-      DualEpi<T> de{K, 0, base_flags, p.num_eq, w.params.p, w.w_table.p, w.y.p, w.y.p, w.q.p,
-                    w.kx.p, w.kx.p, w.anchor_y.p, w.anchor_kx.p, w.dy.p, nullptr, w.sum_y.p,
-                    ylo_ptr};
+    if (cp.ctas > 0) {
+      ClusterStep<T> step{K, 0, p.num_eq, w.params.p, w.w_table.p, w.x.p, w.c.p, w.lo.p, w.hi.p,
+                          w.anchor_x.p, w.dx.p, w.sum_x.p, w.y.p, w.q.p, w.kx.p, w.anchor_y.p,
+                          w.anchor_kx.p, w.dy.p, w.sum_y.p, ylo_ptr,
+                          h_cluster_status.p};
+      const bool stack = K > 1;
+      const int parts = (len + cp.max_len - 1) / cp.max_len;
       if (o.profile) ANU_CUDA(cudaEventRecord(ev_begin, st));
-      launch_cluster_chunk<T>(p, cluster_c, p.dkt.view<T>(), p.dkt.cluster_rows(cluster_c),
-                              p.dk.view<T>(), p.dk.cluster_rows(cluster_c), pe, de, len,
-                              base_flags, base_flags | (check_at_end ? kWriteDelta : 0u));
+      for (int i = 0; i < parts; ++i) {
+        step.it0 = static_cast<int>(static_cast<int64_t>(len) * i / parts);
+        const int end = static_cast<int>(static_cast<int64_t>(len) * (i + 1) / parts);
+        launch_cluster_chunk<T>(p, stack, cp.ctas, cp.threads, p.dkt.view<T>(),
+                                p.dkt.cluster(stack, cp.ctas).rows, p.dk.view<T>(),
+                                p.dk.cluster(stack, cp.ctas).rows, step, end - step.it0, base_flags,
+                                base_flags | (check_at_end && end == len ? kWriteDelta : 0u));
+      }
       return;
     }
     if (o.use_graphs) {
@@ -2207,7 +2262,7 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     for (auto* v : {&vx, &vy, &vc, &vl, &vu, &vq, &oc, &ol, &ou, &oq}) pick(*v);
     K = K2;
     w.K = K2;
-    if (K == 1) cluster_c = cluster_shape<T>(p, o);
+    plan_clusters();
     NK = static_cast<size_t>(std::max(n, 1)) * K;
     MK = static_cast<size_t>(std::max(m, 1)) * K;
     ylo_ptr = any_ylo ? w.ylo.p : nullptr;
@@ -2650,7 +2705,7 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
       }
     }
   }
-  if (persistent) {
+  if (persistent || cp.ctas > 0) {
     ANU_CUDA(cudaStreamSynchronize(st));
     chunks_done();
   }

@@ -171,18 +171,26 @@ struct DevCsr {
   // kSegPerCtaMax segments per CTA).
   void upload(const HostCsr& a, bool with_fp32, cudaStream_t s, int32_t seg_nnz = kSegNnz,
               int32_t seg_per_cta = kSegPerCta);
-  // Row schedules of the cluster-resident single-LP chunk
-  // (cluster_chunk_kernel) for clusters of 16 and of 8 CTAs, and the
-  // longest row; built by prepare_cluster on first use.
-  DevBuf<int32_t> cl_bounds[2], cl_warp_start[2], cl_warp_rows[2];
-  int32_t cl_max_rows[2] = {0, 0}, cl_max_nnz[2] = {0, 0};  // per CTA
-  int32_t max_row = 0;
-  bool cl_ready = false;
-  void prepare_cluster(const HostCsr& a, cudaStream_t s);
+  // Schedules of the cluster-resident chunks (cluster_chunk_kernel), for a
+  // single LP ([0]) and for a case stack ([1]), on clusters of 16 ([][0]) and
+  // of 8 CTAs ([][1]); built by prepare_cluster on first use.
+  struct Cluster {
+    DevBuf<int32_t> bounds, part_start, place, entry;
+    DevBuf<ClusterRow> row;
+    DevBuf<ClusterPart> part;
+    ClusterRows rows{};
+    std::vector<int32_t> row_place;
+    int32_t max_row = 0;
+    bool ready = false;
+  };
+  Cluster clusters[2][2];
+  const Cluster& cluster(bool stack, int ctas) const { return clusters[stack][ctas == 8]; }
+  void prepare_cluster(const HostCsr& a, bool stack, int ctas, int32_t seg_nnz, cudaStream_t s);
+  // Then, once the transpose's schedule is there: where each nonzero's column
+  // sits in the copies of the vector the rows of `other` (the transpose) make.
+  void place_cluster(const HostCsr& a, const Cluster& other, bool stack, int ctas, cudaStream_t s);
   // Selects the single-LP product tile of `threads` (one of kTileThreads).
   void set_tile(int32_t threads);
-  // The cluster schedule for clusters of `ctas` (16 or 8) CTAs.
-  ClusterRows cluster_rows(int ctas) const;
   template <class V>
   CsrView<V> view() const;
 };
@@ -202,6 +210,13 @@ struct Relabel {
 
 // The relabelling of `lp`'s matrix (empty when it has no rows or columns).
 Relabel locality_relabel(const anu_lp& lp);
+
+// How K cases run as cluster-resident chunks: clusters of `ctas` CTAs of
+// `threads`, one per case, at most max_len iterations per launch. ctas 0:
+// they do not.
+struct ClusterPlan {
+  int ctas = 0, threads = 0, max_len = 0;
+};
 
 // Everything that depends on the matrix alone: the scaled matrix and its
 // transpose (host and device), the scaling, ||K~||, the stream.
@@ -227,9 +242,9 @@ struct Problem : Exec {
   // its single-LP checks run on one stream, without a second branch, and
   // launch directly for the first kConcurrentDirect checks of a solve.
   bool concurrent = false;
-  // CTAs per cluster cluster_chunk_kernel runs with on this problem (16, 8,
-  // or 0 where it does not fit); -1 until first asked.
-  int cluster_ctas = -1;
+  // How stacks of so many cases run as cluster-resident chunks, once asked
+  // (cluster_plan).
+  std::map<std::pair<int, int>, ClusterPlan> cluster_plans;
   ~Problem();
 };
 
@@ -275,6 +290,12 @@ std::unique_ptr<Problem> clone_problem(const Problem& src);
 // Case stacks of at least this many cases run as two half-stacks at once,
 // unless they run persistent chunks.
 constexpr int kSplitStack = 16;
+
+// Iterations per cluster-resident launch, unless options.cluster_chunks asks
+// for whole check periods: other streams' clusters wait for a launch to end,
+// so long check periods are cut, and the cut costs little because the next
+// launch loads its matrix slices while the one before still runs.
+constexpr int kClusterLaunchLen = 32;
 
 // Checks a single LP of a packed batch launches directly before its check
 // graphs are captured.

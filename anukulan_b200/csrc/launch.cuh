@@ -213,76 +213,71 @@ void launch_chunk(Exec& p, const Mat& kt, const Mat& k, const T* y, const T* x_b
   ++p.launches;
 }
 
-// ------------------------------------------ cluster-resident single-LP chunks
+// ------------------------------------------------- cluster-resident chunks
 
-// The most dynamic shared memory cluster_chunk_kernel asks for: its copies of
-// y and x_bar and its slices of the two matrices (ClusterLayout).
-constexpr size_t kClusterSmemMax = 200 * 1024;
+// The most dynamic shared memory cluster_chunk_kernel asks for.
+constexpr size_t kClusterSmemMax = 220 * 1024;
 
-// The CTAs per cluster the device runs cluster_chunk_kernel<., T> with: 16
-// where a 16-CTA cluster with smem16 bytes of dynamic shared memory per CTA
-// fits (a non-portable size), else 8 with smem8 bytes, else 0.
 template <class T>
-int cluster_ctas_for(size_t smem16, size_t smem8) {
-  auto fits = [&](auto kernel, int ctas, size_t smem) {
-    if (smem > kClusterSmemMax) return false;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kClusterSmemMax)) != cudaSuccess ||
-        (ctas > 8 &&
-         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-             cudaSuccess)) {
-      cudaGetLastError();
-      return false;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kClusterThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return clusters >= 1;
-  };
-  if (fits(cluster_chunk_kernel<16, T>, 16, smem16)) return 16;
-  if (fits(cluster_chunk_kernel<8, T>, 8, smem8)) return 8;
-  return 0;
+using ClusterKernel = void (*)(CsrView<T>, ClusterRows, CsrView<T>, ClusterRows, ClusterStep<T>,
+                               int32_t, uint32_t, uint32_t);
+template <class T>
+ClusterKernel<T> cluster_kernel(bool stack) {
+  return stack ? cluster_chunk_kernel<T, true> : cluster_chunk_kernel<T, false>;
 }
 
-// `len` iterations of one LP as one launch of one cluster of `ctas` CTAs
-// (from cluster_ctas_for); the schedules must be the ones for that size.
-template <class T>
-void launch_cluster_chunk(Exec& p, int ctas, const CsrView<T>& kt, const ClusterRows& ktr,
-                          const CsrView<T>& k, const ClusterRows& kr, const PrimalEpi<T>& pe,
-                          const DualEpi<T>& de, int len, uint32_t flags, uint32_t last_flags) {
+inline cudaLaunchConfig_t cluster_config(int ctas, int clusters, int threads, size_t smem,
+                                         cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(kClusterThreads);
-  cfg.dynamicSmemBytes = ClusterLayout::of<T>(k.rows, kt.rows, ktr, kr).total;
-  cfg.stream = p.stream;
-  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(ctas * clusters);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ctas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (ctas == 16)
-    cuda_check(cudaLaunchKernelEx(&cfg, cluster_chunk_kernel<16, T>, kt, ktr, k, kr, pe, de, len,
-                                  flags, last_flags),
-               "cluster_chunk_kernel launch");
-  else
-    cuda_check(cudaLaunchKernelEx(&cfg, cluster_chunk_kernel<8, T>, kt, ktr, k, kr, pe, de, len,
-                                  flags, last_flags),
-               "cluster_chunk_kernel launch");
+  cfg.numAttrs = 2;
+  return cfg;
+}
+
+// Clusters of `ctas` CTAs with this much shared memory resident at once; 0
+// where the device does not take them (16 is a non-portable cluster size).
+template <class T>
+int cluster_capacity(ClusterKernel<T> kernel, int ctas, int threads, size_t smem) {
+  if (smem > kClusterSmemMax) return 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(kClusterSmemMax)) != cudaSuccess ||
+      (ctas > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                        1) != cudaSuccess)) {
+    cudaGetLastError();
+    return 0;
+  }
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = cluster_config(ctas, 1, threads, smem, attr);
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters;
+}
+
+// `len` iterations of a stack of step.K cases (or of a single LP) as one launch.
+template <class T>
+void launch_cluster_chunk(Exec& p, bool stack, int ctas, int threads, const CsrView<T>& kt,
+                          const ClusterRows& ktr, const CsrView<T>& k, const ClusterRows& kr,
+                          const ClusterStep<T>& step, int len, uint32_t flags,
+                          uint32_t last_flags) {
+  const size_t smem = ClusterLayout::of<T>(ctas, ktr, kr, len).total;
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = cluster_config(ctas, step.K, threads, smem, attr);
+  cfg.stream = p.stream;
+  cuda_check(cudaLaunchKernelEx(&cfg, cluster_kernel<T>(stack), kt, ktr, k, kr, step, len, flags,
+                                last_flags),
+             "cluster_chunk_kernel launch");
   ++p.launches;
 }
 

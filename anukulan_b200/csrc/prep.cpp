@@ -225,29 +225,87 @@ SegmentSchedule segment_schedule(const HostCsr& a, int32_t seg_nnz, int32_t seg_
   return s;
 }
 
-ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial_row) {
+ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial_row,
+                                 const SegmentSchedule* seg) {
   ClusterSchedule c;
   c.bounds.assign(static_cast<size_t>(parts) + 1, a.rows);
   c.bounds[0] = 0;
-  const int64_t total = a.nnz();
+  const int64_t total = a.nnz() + static_cast<int64_t>(kClusterRowCost) * a.rows;
   int32_t part = 1;
   for (int32_t r = 0; r < a.rows && part < parts; ++r) {
-    // Part `part` starts at the first row whose nonzeros begin at or past
-    // its share; a row never splits.
-    while (part < parts && static_cast<int64_t>(a.start[r]) * parts >= total * part)
-      c.bounds[part++] = r;
+    // Part `part` starts at the first row whose cost begins at or past its
+    // share; a row never splits.
+    const int64_t before = a.start[r] + static_cast<int64_t>(kClusterRowCost) * r;
+    while (part < parts && before * parts >= total * part) c.bounds[part++] = r;
   }
-  c.warp_start.assign(static_cast<size_t>(parts) + 1, 0);
+  c.part_start.push_back(0);
+  c.row.reserve(a.rows);
+  c.entry.resize(a.index.size());
+  constexpr int32_t kLanes = 32;
   for (int32_t q = 0; q < parts; ++q) {
-    for (int32_t r = c.bounds[q]; r < c.bounds[q + 1]; ++r) {
-      const int32_t len = a.start[r + 1] - a.start[r];
+    const int32_t rb = c.bounds[q], re = c.bounds[q + 1];
+    const size_t p0 = c.part.size();
+    int32_t slots = 0;
+    // Here `first` is the sum's first nonzero; the layout below replaces it.
+    for (int32_t r = rb; r < re; ++r) {
+      const int32_t b = a.start[r], len = a.start[r + 1] - b;
       c.max_row = std::max(c.max_row, len);
-      if (len > serial_row) c.warp_rows.push_back(r);
+      const int32_t g0 = seg != nullptr ? seg->row_seg[r] : 0;
+      const int32_t g1 = seg != nullptr ? seg->row_seg[r + 1] : (len > serial_row ? 2 : 1);
+      if (g1 - g0 <= 1) {
+        c.row.push_back({r, b, len, 0});
+      } else if (seg == nullptr) {
+        c.row.push_back({r, slots, 1, 1});
+        c.part.push_back({b, len, slots++});
+      } else {
+        c.row.push_back({r, slots, g1 - g0, 1});
+        for (int32_t g = g0; g < g1; ++g) {
+          const int32_t e = g + 1 < g1 ? seg->seg_begin[g + 1] : a.start[r + 1];
+          c.part.push_back({seg->seg_begin[g], e - seg->seg_begin[g], slots++});
+        }
+      }
     }
-    c.warp_start[q + 1] = static_cast<int32_t>(c.warp_rows.size());
-    c.max_part_rows = std::max(c.max_part_rows, c.bounds[q + 1] - c.bounds[q]);
-    c.max_part_nnz = std::max(c.max_part_nnz, a.start[c.bounds[q + 1]] - a.start[c.bounds[q]]);
+    std::stable_sort(c.row.begin() + rb, c.row.begin() + re,
+                     [](const ClusterSchedule::Row& x, const ClusterSchedule::Row& y) {
+                       return (x.apart ? 0 : x.count) > (y.apart ? 0 : y.count);
+                     });
+    int32_t entries = 0;
+    auto lay_out = [&](int32_t* first, int32_t count, int32_t at, int32_t step) {
+      for (int32_t k = 0; k < count; ++k) c.entry[*first + k] = at + k * step;
+      *first = at;
+    };
+    // Thread-summed: the i-th row (or segment) in lane i % 32 of its group.
+    auto lanes = [&](auto&& get, int32_t count) {
+      for (int32_t i0 = 0; i0 < count; i0 += kLanes) {
+        int32_t longest = 0;
+        for (int32_t i = i0; i < std::min(count, i0 + kLanes); ++i) {
+          auto* d = get(i);
+          if (d == nullptr) continue;
+          longest = std::max(longest, d->count);
+          lay_out(&d->first, d->count, entries + i - i0, kLanes);
+        }
+        entries += longest * kLanes;
+      }
+    };
+    lanes([&](int32_t i) { return c.row[rb + i].apart ? nullptr : &c.row[rb + i]; }, re - rb);
+    if (seg != nullptr) {
+      lanes([&](int32_t i) { return &c.part[p0 + i]; }, static_cast<int32_t>(c.part.size() - p0));
+    } else {
+      for (size_t i = p0; i < c.part.size(); ++i) {
+        lay_out(&c.part[i].first, c.part[i].count, entries, 1);
+        entries += c.part[i].count;
+      }
+    }
+    c.part_start.push_back(static_cast<int32_t>(c.part.size()));
+    c.max_rows = std::max(c.max_rows, re - rb);
+    c.max_entries = std::max(c.max_entries, entries);
+    c.max_parts = std::max(c.max_parts, slots);
   }
+  c.stride = (c.max_rows + 3) / 4 * 4;
+  c.place.resize(a.rows);
+  for (int32_t q = 0; q < parts; ++q)
+    for (int32_t r = c.bounds[q]; r < c.bounds[q + 1]; ++r)
+      c.place[c.row[r].row] = q * c.stride + (r - c.bounds[q]);
   return c;
 }
 

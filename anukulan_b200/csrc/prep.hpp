@@ -90,18 +90,36 @@ SegmentSchedule segment_schedule(const HostCsr& a, int32_t seg_nnz, int32_t seg_
                                  int32_t row_max);
 
 // The rows of a matrix dealt to the `parts` CTAs of one thread-block cluster
-// (see cluster_chunk_kernel): contiguous ranges, cut where the running
-// nonzero count crosses each part's even share. Rows of more than
-// serial_row nonzeros are summed by a warp; each part lists its own.
+// (see cluster_chunk_kernel): contiguous ranges, cut where the running cost
+// (a row's nonzeros plus kClusterRowCost for its step) crosses each part's
+// even share, each row's sum, and the sums taken apart from the row's owner:
+//  - stack: the segments of `seg`, for rows of several;
+//  - single LP (seg null): whole rows of more than serial_row nonzeros.
+// The nonzeros of a part are laid out for its threads: those a thread sums 32
+// entries apart, beside those of the warp's other lanes (rows go to threads
+// longest first, so lanes of a warp hold rows of like length), those a warp
+// sums one after another. Entries and partial sums are counted from the part's
+// first.
 struct ClusterSchedule {
+  struct Row {
+    int32_t row, first, count, apart;
+  };
+  struct Part {
+    int32_t first, count, slot;
+  };
   std::vector<int32_t> bounds;      // parts + 1 row bounds
-  std::vector<int32_t> warp_start;  // parts + 1 offsets into warp_rows
-  std::vector<int32_t> warp_rows;   // the rows longer than serial_row, by part
-  int32_t max_row = 0;              // longest row
-  int32_t max_part_rows = 0;        // most rows in one part
-  int32_t max_part_nnz = 0;         // most nonzeros in one part
+  std::vector<int32_t> part_start;  // parts + 1
+  std::vector<Row> row;       // by part; within it the longest own sums first
+  std::vector<Part> part;
+  std::vector<int32_t> place;  // of each row: part * stride + its position in the part
+  std::vector<int32_t> entry;  // of each nonzero, in its part's layout
+  int32_t stride = 0;          // max_rows in whole 16-byte groups
+  int32_t max_row = 0;  // the longest row
+  int32_t max_rows = 0, max_entries = 0, max_parts = 0;  // the most one part holds
 };
-ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial_row);
+constexpr int32_t kClusterRowCost = 4;
+ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial_row,
+                                 const SegmentSchedule* seg);
 
 double now_seconds();
 
