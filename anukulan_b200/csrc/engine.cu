@@ -976,8 +976,7 @@ struct Workspace {
   // scaled data the correction LPs are formed from, K times a column shift,
   // and the averaged scheme's running weight per case
   DevBuf<double> xb, yb, x_comb, y_comb, c0s, q0s, l0s, u0s, kshift, sum_weight;
-  DevBuf<StepParams> params;
-  DevBuf<double> w_table;
+  DevBuf<double> step_data;
   DevBuf<int32_t> mask;
   DevBuf<double> partial, partial2, terms, kkt, weights;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
@@ -1506,15 +1505,22 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     upload_interleaved(st, w.l0s, n, K, vl);
     upload_interleaved(st, w.u0s, n, K, vu);
   }
-  w.params.alloc(K);
   w.mask.alloc(K);
   w.terms.alloc(static_cast<size_t>(kCheckTerms) * K * 2);
   w.kkt.alloc(static_cast<size_t>(kKktTerms) * K * 2);
   w.weights.alloc(K);
   const int F = o.termination_check_frequency;
-  w.w_table.alloc(static_cast<size_t>(std::max(F, 1)) * K);
-  Pinned<StepParams> h_params(K);
-  Pinned<double> h_w(static_cast<size_t>(std::max(F, 1)) * K);
+  // The cases' step parameters and, behind them, the chunk's Halpern weights:
+  // one buffer, one upload per chunk.
+  static_assert(sizeof(StepParams) % sizeof(double) == 0, "weights follow the parameters");
+  const size_t params_doubles = sizeof(StepParams) / sizeof(double) * K;
+  const size_t step_doubles = params_doubles + static_cast<size_t>(std::max(F, 1)) * K;
+  w.step_data.alloc(step_doubles);
+  Pinned<double> h_step(step_doubles);
+  StepParams* const h_params = reinterpret_cast<StepParams*>(h_step.p);
+  double* h_w = h_step.p + params_doubles;
+  const StepParams* const d_params = reinterpret_cast<const StepParams*>(w.step_data.p);
+  const double* d_w = w.step_data.p + params_doubles;
   Pinned<double> h_terms(static_cast<size_t>(kCheckTerms) * K * 2);
   Pinned<double> h_kkt(static_cast<size_t>(kKktTerms) * K * 2);
   // Case masks go up through a ring of pinned staging slots, so a new mask
@@ -1564,7 +1570,7 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
   // Per-chunk parameter upload.
   auto upload_params = [&](int len) {
     for (int k = 0; k < K; ++k) {
-      StepParams& P = h_params.p[k];
+      StepParams& P = h_params[k];
       P.tau = S[k].eta / S[k].omega;
       P.sigma = S[k].eta * S[k].omega;
       P.gamma = reflection;
@@ -1580,21 +1586,22 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
           if (!(P.reset_pending && it == 0))
             wv = static_cast<double>(kk + 1) / static_cast<double>(kk + 2);
         }
-        h_w.p[static_cast<size_t>(it) * K + k] = wv;
+        h_w[static_cast<size_t>(it) * K + k] = wv;
       }
     }
-    ANU_CUDA(cudaMemcpyAsync(w.params.p, h_params.p, sizeof(StepParams) * K, cudaMemcpyHostToDevice, st));
-    ANU_CUDA(cudaMemcpyAsync(w.w_table.p, h_w.p, sizeof(double) * len * K, cudaMemcpyHostToDevice, st));
+    ANU_CUDA(cudaMemcpyAsync(w.step_data.p, h_step.p,
+                             sizeof(double) * (d_w - w.step_data.p) + sizeof(double) * len * K,
+                             cudaMemcpyHostToDevice, st));
   };
 
   const T* ylo_ptr = any_ylo ? w.ylo.p : nullptr;
 
   // One fast-path iteration (in place).
   auto launch_iteration = [&](int it, uint32_t flags) {
-    PrimalEpi<T> pe{K, it, flags, w.params.p, w.w_table.p, w.x.p, w.x.p, w.c.p, w.lo.p, w.hi.p,
+    PrimalEpi<T> pe{K, it, flags, d_params, d_w, w.x.p, w.x.p, w.c.p, w.lo.p, w.hi.p,
                     w.x_bar.p, w.anchor_x.p, w.dx.p, w.sum_x.p};
     product<T, T, T>(p, p.dkt, w.y.p, K, pe, true);
-    DualEpi<T> de{K, it, flags, p.num_eq, w.params.p, w.w_table.p, w.y.p, w.y.p, w.q.p, w.kx.p,
+    DualEpi<T> de{K, it, flags, p.num_eq, d_params, d_w, w.y.p, w.y.p, w.q.p, w.kx.p,
                   w.kx.p, w.anchor_y.p, w.anchor_kx.p, w.dy.p, nullptr, w.sum_y.p, ylo_ptr};
     product<T, T, T>(p, p.dk, w.x_bar.p, K, de, true);
   };
@@ -1684,9 +1691,9 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     if (persistent) {
       if (!coop_lock.owns_lock()) coop_lock.lock();
       if (o.profile) ANU_CUDA(cudaEventRecord(ev_begin, st));
-      PrimalEpi<T> pe{K, 0, 0u, w.params.p, w.w_table.p, w.x.p, w.x.p, w.c.p, w.lo.p, w.hi.p,
+      PrimalEpi<T> pe{K, 0, 0u, d_params, d_w, w.x.p, w.x.p, w.c.p, w.lo.p, w.hi.p,
                       w.x_bar.p, w.anchor_x.p, w.dx.p, w.sum_x.p};
-      DualEpi<T> de{K, 0, 0u, p.num_eq, w.params.p, w.w_table.p, w.y.p, w.y.p, w.q.p, w.kx.p,
+      DualEpi<T> de{K, 0, 0u, p.num_eq, d_params, d_w, w.y.p, w.y.p, w.q.p, w.kx.p,
                     w.kx.p, w.anchor_y.p, w.anchor_kx.p, w.dy.p, nullptr, w.sum_y.p, ylo_ptr};
       ANU_CUDA(cudaMemsetAsync(sync_arrived.p, 0, sizeof(uint32_t), st));
       launch_chunk<T>(p, p.dkt, p.dk, w.y.p, w.x_bar.p, K, len, base_flags,
@@ -1697,7 +1704,7 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
       return;
     }
     if (cp.ctas > 0) {
-      ClusterStep<T> step{K, 0, p.num_eq, w.params.p, w.w_table.p, w.x.p, w.c.p, w.lo.p, w.hi.p,
+      ClusterStep<T> step{K, 0, p.num_eq, d_params, d_w, w.x.p, w.c.p, w.lo.p, w.hi.p,
                           w.anchor_x.p, w.dx.p, w.sum_x.p, w.y.p, w.q.p, w.kx.p, w.anchor_y.p,
                           w.anchor_kx.p, w.dy.p, w.sum_y.p, ylo_ptr,
                           h_cluster_status.p};
@@ -1893,7 +1900,10 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     p.launches += r.launches;
   };
 
+  std::vector<int32_t> mask_now;  // what w.mask holds; empty before the first upload
   auto set_mask = [&](const std::vector<int32_t>& mk) {
+    if (mk == mask_now) return;
+    mask_now = mk;
     // Wrapping around the ring, the slot about to be refilled may still feed
     // a copy: drain the stream first.
     mask_slot = (mask_slot + 1) % kMaskSlots;
@@ -1963,6 +1973,11 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
       if (mk[k]) ++R_ptr->at(orig[k]).r.refinement_rounds;
   };
 
+  struct ChunkEnd {
+    cudaEvent_t event = nullptr;
+    ChunkEnd() { ANU_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming)); }
+    ~ChunkEnd() { cudaEventDestroy(event); }
+  } chunk_end;
   int32_t iteration = 0;
   std::vector<CaseResult>& R = *results;
   for (int k = 0; k < K; ++k) {
@@ -2262,6 +2277,9 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     for (auto* v : {&vx, &vy, &vc, &vl, &vu, &vq, &oc, &ol, &ou, &oq}) pick(*v);
     K = K2;
     w.K = K2;
+    // The weights follow the parameters of the cases that are left.
+    h_w = h_step.p + sizeof(StepParams) / sizeof(double) * K;
+    d_w = w.step_data.p + sizeof(StepParams) / sizeof(double) * K;
     plan_clusters();
     NK = static_cast<size_t>(std::max(n, 1)) * K;
     MK = static_cast<size_t>(std::max(m, 1)) * K;
@@ -2314,7 +2332,7 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
       const double hw = blend ? static_cast<double>(c.halpern_k + 1) / static_cast<double>(c.halpern_k + 2) : 1.0;
       const bool need_movement = adaptive || o.halpern_restart || is_check;
       for (int attempt = 0;; ++attempt) {
-        StepParams& P = h_params.p[0];
+        StepParams& P = h_params[0];
         P.tau = c.eta / c.omega;
         P.sigma = c.eta * c.omega;
         P.gamma = reflection;
@@ -2323,13 +2341,13 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
         P.halpern = blend ? 1 : 0;
         P.reset_pending = 0;
         P.k_base = 0;
-        h_w.p[0] = hw;
-        ANU_CUDA(cudaMemcpyAsync(w.params.p, h_params.p, sizeof(StepParams), cudaMemcpyHostToDevice, st));
-        ANU_CUDA(cudaMemcpyAsync(w.w_table.p, h_w.p, sizeof(double), cudaMemcpyHostToDevice, st));
-        PrimalEpi<T> pe{1, 0, kWriteDelta, w.params.p, w.w_table.p, w.x.p, w.x_next.p, w.c.p,
+        h_w[0] = hw;
+        ANU_CUDA(cudaMemcpyAsync(w.step_data.p, h_step.p, sizeof(double) * (params_doubles + 1),
+                                 cudaMemcpyHostToDevice, st));
+        PrimalEpi<T> pe{1, 0, kWriteDelta, d_params, d_w, w.x.p, w.x_next.p, w.c.p,
                         w.lo.p, w.hi.p, w.x_bar.p, w.anchor_x.p, w.dx.p, nullptr};
         product<T, T, T>(p, p.dkt, w.y.p, 1, pe);
-        DualEpi<T> de{1, 0, kWriteDelta, p.num_eq, w.params.p, w.w_table.p, w.y.p, w.y_next.p,
+        DualEpi<T> de{1, 0, kWriteDelta, p.num_eq, d_params, d_w, w.y.p, w.y_next.p,
                       w.q.p, w.kx.p, w.k_next.p, w.anchor_y.p, w.anchor_kx.p, w.dy.p, w.k_dx.p,
                       nullptr, ylo_ptr};
         product<T, T, T>(p, p.dk, w.x_bar.p, 1, de);
@@ -2397,9 +2415,17 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     }
     iteration = last + 1;
     if (!is_check) continue;
-    ANU_CUDA(cudaStreamSynchronize(st));
-    chunks_done();
-    t_iter += phase_end();
+    // The check is queued behind the chunk at once; the host waits for the
+    // chunk's end (chunk_end) only then, so the device goes from one to the
+    // other without it. Not where the check itself waits on the way.
+    const bool wait_first = slow || persistent || need_kkt_any || averaging;
+    if (wait_first) {
+      ANU_CUDA(cudaStreamSynchronize(st));
+      chunks_done();
+      t_iter += phase_end();
+    } else {
+      ANU_CUDA(cudaEventRecord(chunk_end.event, st));
+    }
 
     // ------------------------------------------------------------- check
     const int32_t it_idx = last;
@@ -2428,6 +2454,11 @@ void run_cases_t(Problem& p, const std::vector<const CaseData*>& initial_cases,
     if (need_kkt || any_avg)
       ANU_CUDA(cudaMemcpyAsync(h_kkt.p, w.kkt.p, sizeof(double) * kKktTerms * K * (any_avg ? 2 : 1),
                                cudaMemcpyDeviceToHost, st));
+    if (!wait_first) {
+      ANU_CUDA(cudaEventSynchronize(chunk_end.event));
+      chunks_done();
+      t_iter += phase_end();
+    }
     ANU_CUDA(cudaStreamSynchronize(st));
     collect_chunk_time();
 
