@@ -83,9 +83,9 @@ struct UnrollPrimal {
   struct Pre {
     T c, lo, hi, tau, x, anchor;
   };
-  // On a case stack the launches are long enough to hide their own loads, and
-  // items held ahead cost registers: 18.0 ms per 60-case, 300-step forward and
-  // backward without, 19.8 ms with two ahead.
+  // seg_kernel's items are not loaded ahead: beside these epilogues the
+  // registers cost more than the latency (15.4 ms per 60-case, 300-step forward
+  // and backward, 19.8 ms with two ahead).
   static constexpr int kPrefetch = 0;
   __device__ __forceinline__ Pre prefetch(int32_t row, int32_t k) const {
     Pre r;
@@ -107,7 +107,7 @@ struct UnrollPrimal {
     if (!restart) r.anchor = anchor[e];
   }
   __device__ __forceinline__ void finish(int32_t j, int32_t k, T kty, const Pre& r,
-                                         NoParams) const {
+                                         NoParams = {}) const {
     const size_t e = static_cast<size_t>(j) * K + k;
     const T xj = r.x;
     const T u = sub(xj, mul(r.tau, sub(r.c, kty)));
@@ -159,7 +159,7 @@ struct UnrollDual {
     if (!restart) r.anchor = anchor[e];
   }
   __device__ __forceinline__ void finish(int32_t i, int32_t k, T bar, const Pre& r,
-                                         NoParams) const {
+                                         NoParams = {}) const {
     const size_t e = static_cast<size_t>(i) * K + k;
     const T yi = r.y;
     const T s = add(yi, mul(r.sigma, sub(r.q, bar)));
@@ -249,7 +249,7 @@ struct RevPrimal {
     r.grad = gc[e];
   }
   __device__ __forceinline__ void finish(int32_t j, int32_t k, T ktz, const Pre& r,
-                                         NoParams) const {
+                                         NoParams = {}) const {
     const size_t e = static_cast<size_t>(j) * K + k;
     const T xplus = r.x;
     T m;
@@ -310,7 +310,7 @@ struct RevDual {
     }
   }
   __device__ __forceinline__ void finish(int32_t i, int32_t k, T kuh, const Pre& r,
-                                         NoParams) const {
+                                         NoParams = {}) const {
     const size_t e = static_cast<size_t>(i) * K + k;
     const T yt = add(r.y, mul(r.tau, kuh));
     if (mask_prev == nullptr) {
@@ -449,11 +449,11 @@ void forward_step(Problem& p, int K, UnrollState<T>& s, int t, int period, uint8
   product<T, T, T>(p, p.dkt, s.y.p, K,
                    UnrollPrimal<T>{K, s.tau.p, sc.restart ? 1 : 0, sc.a, s.x.p, s.c.p, s.lo.p,
                                    s.hi.p, s.ax.p, s.x_bar.p, mx},
-                   K == 1);
+                   true);
   product<T, T, T>(p, p.dk, s.x_bar.p, K,
                    UnrollDual<T>{K, p.num_eq, s.sigma.p, sc.restart ? 1 : 0, sc.a, s.y.p, s.q.p,
                                  s.ay.p, my},
-                   K == 1);
+                   true);
 }
 
 // Copies the state (x, y, ax, ay) into or out of checkpoint slot `seg`.
@@ -588,14 +588,14 @@ void backward_t(Unrolled& u, UnrollState<T>& s, const double* dx, const double* 
         product<T, T, T>(p, p.dkt, z.p, K,
                          RevPrimal<T>{K, s.tau.p, sj.restart ? 1 : 0, sj.a, xh.p, axh.p,
                                       mx.p + static_cast<size_t>(j) * s.nk, uh.p, gc.p},
-                         K == 1);
+                         true);
         const bool more = j > 0;
         const StepSchedule sp = more ? schedule(j - 1, R) : StepSchedule{false, 0.0};
         product<T, T, T>(p, p.dk, uh.p, K,
                          RevDual<T>{K, s.tau.p, s.sigma.p, yh.p, ayh.p, z.p, gq.p,
                                     more ? my.p + static_cast<size_t>(j - 1) * s.mk : nullptr,
                                     sp.restart ? 1 : 0, sp.a},
-                         K == 1);
+                         true);
       }
     };
     if (len == R) {
