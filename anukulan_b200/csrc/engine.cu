@@ -364,7 +364,7 @@ template <class T>
 struct SquareTerms {
   static constexpr int NT = 1;
   int32_t K;
-  const T* __restrict__ v;
+  const T* v;
   __device__ static void init(double* a) { a[0] = 0.0; }
   __device__ static double identity(int) { return 0.0; }
   __device__ static double combine(int, double a, double b) { return anu::add(a, b); }
@@ -390,9 +390,11 @@ struct StepRowTerms {
   }
 };
 
-__global__ void normalize_kernel(int32_t n, const double* __restrict__ in,
-                                 const double* __restrict__ sumsq, double* __restrict__ out,
+__global__ void normalize_kernel(int32_t n, const double* in,
+                                 const double* sumsq, double* __restrict__ out,
                                  double* __restrict__ estimates, int32_t slot) {
+  pdl_launch();
+  pdl_wait();
   const double next = sqrt(sumsq[0]);
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * blockDim.x)
@@ -436,13 +438,12 @@ double device_matrix_norm(Problem& p, int iterations, double tolerance) {
   std::vector<double> h_est(chunk);
   auto enqueue = [&](int count) {
     for (int it = 0; it < count; ++it) {
-      product<double, double, double>(p, p.dk, dv.p, 1, StoreEpi<double>{1, dkv.p});
-      product<double, double, double>(p, p.dkt, dkv.p, 1, StoreEpi<double>{1, dktkv.p});
-      reduce_terms(p, n, 1, SquareTerms<double>{1, dktkv.p}, partial, sumsq.p, 1, 0);
-      normalize_kernel<<<grid_for(n, 256, 296), 256, 0, p.stream>>>(n, dktkv.p, sumsq.p, dv.p,
-                                                                     est.p, it);
-      ANU_CUDA(cudaGetLastError());
-      ++p.launches;
+      product<double, double, double>(p, p.dk, dv.p, 1, StoreEpi<double>{1, dkv.p}, true);
+      product<double, double, double>(p, p.dkt, dkv.p, 1, StoreEpi<double>{1, dktkv.p}, true);
+      reduce_terms(p, n, 1, SquareTerms<double>{1, dktkv.p}, partial, sumsq.p, 1, 0, true);
+      launch_dependent(p, grid_for(n, 256, 296), 256, normalize_kernel, n,
+                       static_cast<const double*>(dktkv.p), static_cast<const double*>(sumsq.p),
+                       dv.p, est.p, it);
     }
   };
   struct GraphGuard {

@@ -1206,6 +1206,69 @@ __global__ void terms_stage2(int32_t blocks, int32_t K, const double* __restrict
   if (lane == 0) out[(size_t)k * stride + offset + q] = acc;
 }
 
+// Both stages for a single case in one launch. The check of a small LP is a
+// chain of launches of a few microseconds each, so the last block to finish
+// (counted in `arrived`, which it leaves at zero for the next launch) folds the
+// blocks' partials instead of a second launch, and a block's tree takes one
+// barrier: its three widest levels are folded by the warp that owns a term, the
+// rest by shuffles. Every pair is combined as the two stages combine it, in the
+// same order, so the results are the same bit for bit. A check through the
+// backend seam on a 37,501 x 56,251 LP (two products, two reductions and the
+// read-back): 54.5 us with two launches per reduction, 51 with one.
+template <class Terms>
+__global__ void __launch_bounds__(kThreads) terms_single(int32_t len, Terms t,
+                                                         double* __restrict__ partial,
+                                                         unsigned* __restrict__ arrived,
+                                                         double* __restrict__ out) {
+  constexpr int NT = Terms::NT;
+  constexpr int kWarps = kThreads / 32;
+  static_assert(kWarps == 8, "the folds below are for eight warps");
+  __shared__ double red[kWarps][NT][32];
+  __shared__ bool last;
+  pdl_launch();
+  pdl_wait();
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  double acc[NT];
+  Terms::init(acc);
+  for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < len;
+       r += (int64_t)gridDim.x * kThreads)
+    t.add(acc, static_cast<int32_t>(r), 0);
+#pragma unroll
+  for (int q = 0; q < NT; ++q) red[warp][q][lane] = acc[q];
+  __syncthreads();
+  for (int q = warp; q < NT; q += kWarps) {
+    double v[kWarps];
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) v[w] = red[w][q][lane];
+#pragma unroll
+    for (int s = kWarps / 2; s > 0; s >>= 1)
+#pragma unroll
+      for (int w = 0; w < s; ++w) v[w] = Terms::combine(q, v[w], v[w + s]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+      v[0] = Terms::combine(q, v[0], __shfl_down_sync(0xffffffffu, v[0], off));
+    if (lane == 0) {
+      partial[(size_t)blockIdx.x * NT + q] = v[0];
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int q = warp; q < NT; q += kWarps) {
+    double v = Terms::identity(q);
+    for (int32_t b = lane; b < static_cast<int32_t>(gridDim.x); b += 32)
+      v = Terms::combine(q, v, __ldcg(partial + (size_t)b * NT + q));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+      v = Terms::combine(q, v, __shfl_down_sync(0xffffffffu, v, off));
+    if (lane == 0) out[q] = v;
+  }
+  if (threadIdx.x == 0) *arrived = 0u;
+}
+
 // ------------------------------------------------------------ check terms
 
 // Row side of a termination check, per case (backend.cpp:143-161 and the

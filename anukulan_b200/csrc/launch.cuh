@@ -281,23 +281,62 @@ void launch_cluster_chunk(Exec& p, bool stack, int ctas, int threads, const CsrV
   ++p.launches;
 }
 
-// Two-stage per-case reduction of `t` over len rows; results land in
+// A kernel launch that may start while its predecessor in the stream runs (see
+// pdl_wait).
+template <class... Params, class... Args>
+void launch_dependent(Exec& p, int grid, int threads, void (*kernel)(Params...), Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = p.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cuda_check(cudaLaunchKernelEx(&cfg, kernel, args...), "kernel launch");
+  ++p.launches;
+}
+
+// Reduction scratch for `count` partials, and behind them the arrival counter
+// of terms_single, which is zero between launches.
+template <class Buf>
+void reserve_partials(Exec& p, Buf& partial, size_t count) {
+  if (partial.n > count) return;
+  partial.alloc(count + 1);
+  cuda_check(cudaMemsetAsync(partial.p + count, 0, sizeof(double), p.stream),
+             "cudaMemsetAsync");
+}
+
+// Per-case reduction of `t` over len rows; results land in
 // out[case*stride + offset + term] (device).
 template <class Terms, class Buf>
 void reduce_terms(Exec& p, int32_t len, int K, const Terms& t, Buf& partial,
-                  double* out, int stride, int offset) {
+                  double* out, int stride, int offset, bool pdl = false) {
   constexpr int NT = Terms::NT;
   cudaStream_t s = p.stream;
   int blocks = 0;
+  if (K == 1) {
+    blocks = grid_for(len, kThreads, 296);
+    reserve_partials(p, partial, static_cast<size_t>(blocks) * NT);
+    unsigned* arrived = reinterpret_cast<unsigned*>(partial.p + partial.n - 1);
+    if (pdl) {
+      launch_dependent(p, blocks, kThreads, terms_single<Terms>, len, t, partial.p, arrived,
+                       out + offset);
+      return;
+    }
+    terms_single<Terms><<<blocks, kThreads, 0, s>>>(len, t, partial.p, arrived, out + offset);
+    cuda_check(cudaGetLastError(), "kernel launch");
+    ++p.launches;
+    return;
+  }
 #define ANU_TERMS(L_, CPL_)                                                           \
   do {                                                                                \
     blocks = grid_for(len, kThreads / L_, 296);                                       \
-    if (partial.n < static_cast<size_t>(blocks) * K * NT)                             \
-      partial.alloc(static_cast<size_t>(blocks) * K * NT);                            \
+    reserve_partials(p, partial, static_cast<size_t>(blocks) * K * NT);               \
     terms_stage1<Terms, L_, CPL_><<<blocks, kThreads, 0, s>>>(len, K, t, partial.p);  \
   } while (0)
-  if (K == 1) ANU_TERMS(1, 1);
-  else if (K <= 4) ANU_TERMS(4, 1);
+  if (K <= 4) ANU_TERMS(4, 1);
   else if (K <= 8) ANU_TERMS(8, 1);
   else if (K <= 16) ANU_TERMS(16, 1);
   else if (K <= 32) ANU_TERMS(32, 1);
