@@ -60,7 +60,7 @@ namespace anu {
 // The longest launch: its Halpern weights sit in shared memory.
 constexpr int kClusterMaxLen = 1024;
 // The most threads, hence rows of either matrix, per CTA.
-constexpr int kClusterThreadsMax = 512;
+constexpr int kClusterThreadsMax = 1024;
 // Clock cycles (about a second) before a wait gives up.
 constexpr long long kClusterPatience = 1ll << 31;
 

@@ -1220,7 +1220,8 @@ ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   ClusterPlan none;
   if (p.m == 0 || p.n == 0 || p.dk.nnz == 0) return none;
   // Before any schedule is built: the shares are even at best.
-  if (std::max(p.m, p.n) > 16 * kClusterThreadsMax ||
+  const int most = p.concurrent ? kClusterThreadsMax : kClusterThreadsAlone;
+  if (std::max(p.m, p.n) > 16 * most ||
       2 * sizeof(ClusterNz<T>) * (p.dk.nnz / 16) + sizeof(T) * (p.m + p.n) > kClusterSmemMax)
     return none;
   const auto key = std::make_pair(K, max_len);
@@ -1234,12 +1235,12 @@ ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
     const DevCsr::Cluster &ck = p.dk.cluster(stack, ctas), &ckt = p.dkt.cluster(stack, ctas);
     if (!stack && std::max(ck.max_row, ckt.max_row) > kLongRow) break;
     const int32_t rows = std::max(ck.rows.max_rows, ckt.rows.max_rows);
-    if (rows > kClusterThreadsMax) break;
+    if (rows > most) break;
     // Threads for the rows, and as far as there is room for the sums apart
     // beside them: a warp each for a single LP, a thread each for a stack.
     const int32_t parts = std::max(ck.rows.max_parts, ckt.rows.max_parts);
     const int32_t want = std::max(128, stack ? rows + parts : std::max(rows, 32 * parts));
-    const int threads = std::min((want + 31) / 32 * 32, kClusterThreadsMax);
+    const int threads = std::min((want + 31) / 32 * 32, std::max<int32_t>(kClusterThreadsAlone, (rows + 31) / 32 * 32));
     const size_t smem = ClusterLayout::of<T>(ctas, ckt.rows, ck.rows, max_len).total;
     if (cluster_capacity<T>(cluster_kernel<T>(stack), ctas, threads, smem) < K) continue;
     p.dk.place_cluster(p.k, ckt, stack, ctas, p.stream);

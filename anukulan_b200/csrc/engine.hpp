@@ -291,6 +291,11 @@ std::unique_ptr<Problem> clone_problem(const Problem& src);
 // unless they run persistent chunks.
 constexpr int kSplitStack = 16;
 
+// The most threads per CTA, hence sixteenths of a matrix's rows and columns,
+// for a problem that has the device to itself. A larger matrix is quicker over
+// the whole device then; one of a packed batch shares it and takes clusters up
+// to kClusterThreadsMax.
+constexpr int kClusterThreadsAlone = 512;
 // Iterations per cluster-resident launch, unless options.cluster_chunks asks
 // for whole check periods: other streams' clusters wait for a launch to end,
 // so long check periods are cut, and the cut costs little because the next
