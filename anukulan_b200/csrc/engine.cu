@@ -1211,10 +1211,15 @@ void run_polish(Problem& p, bool unit, const std::vector<const CaseData*>& paren
 }
 
 // How K cases on `p` run as cluster-resident chunks (cluster_chunk_kernel):
-// clusters of 16 CTAs (8 where the device takes no cluster of 16), all of them
-// resident at once. Not taken where a CTA's rows exceed its threads or its
-// slices its shared memory, where a single LP has a row longer than kLongRow (which more
-// than a warp sums), or where the clusters would have to take turns.
+// clusters of 16 CTAs (8 where the device takes no cluster of 16), one per
+// case. Not taken where a CTA's rows exceed its threads or its slices its
+// shared memory, where a single LP has a row longer than kLongRow (which more
+// than a warp sums), or where the stack needs more than four clusters for
+// every three that are resident at once: the others wait their turn, and a
+// stack of launches that each carry every case is quicker from there on (400
+// iterations of a 24-period refinery stack in FP32, 15 clusters resident, as
+// two half-stacks: 32 cases 10.8 ms against 12.3, 40 cases 13.1 against 13.5;
+// in FP64, 7 resident, one stack of 8: 6.1 against 7.8).
 template <class T>
 ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   ClusterPlan none;
@@ -1242,7 +1247,8 @@ ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
     const int32_t want = std::max(128, stack ? rows + parts : std::max(rows, 32 * parts));
     const int threads = std::min((want + 31) / 32 * 32, std::max<int32_t>(kClusterThreadsAlone, (rows + 31) / 32 * 32));
     const size_t smem = ClusterLayout::of<T>(ctas, ckt.rows, ck.rows, max_len).total;
-    if (cluster_capacity<T>(cluster_kernel<T>(stack), ctas, threads, smem) < K) continue;
+    const int resident = cluster_capacity<T>(cluster_kernel<T>(stack), ctas, threads, smem);
+    if (3 * K > 4 * resident) continue;
     p.dk.place_cluster(p.k, ckt, stack, ctas, p.stream);
     p.dkt.place_cluster(p.kt, ck, stack, ctas, p.stream);
     plan = {ctas, threads, max_len};
