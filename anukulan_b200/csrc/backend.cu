@@ -162,13 +162,21 @@ int guard(F&& body) {
   }
 }
 
+// The products and the two updates are dependent launches (pdl_wait): queued
+// one after another, as an iteration queues them, each one's launch and a
+// product's index loads run beside the one before (an iteration of a 200,000 x
+// 300,000 LP 48.4 -> 38.8 us). Their vectors may be what that one writes, so
+// they are read after the wait and with plain loads. The other operations are
+// plain launches and wait for everything before them.
+
 // backend.cpp:60-79, one thread per entry, no FMA contraction.
 __global__ void primal_update_kernel(int64_t n, double tau, double gamma, double halpern,
-                                     const double* x, const double* __restrict__ c,
-                                     const double* __restrict__ kt_y,
-                                     const double* __restrict__ lower,
-                                     const double* __restrict__ upper, const double* anchor,
+                                     const double* x, const double* c, const double* kt_y,
+                                     const double* lower, const double* upper,
+                                     const double* anchor,
                                      double* x_out, double* dx, double* x_bar) {
+  pdl_launch();
+  pdl_wait();
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * blockDim.x) {
     const double xj = x[j];
@@ -188,10 +196,12 @@ __global__ void primal_update_kernel(int64_t n, double tau, double gamma, double
 
 // backend.cpp:81-111.
 __global__ void dual_update_kernel(int64_t m, int64_t num_eq, double sigma, double gamma,
-                                   double halpern, const double* y, const double* __restrict__ q,
+                                   double halpern, const double* y, const double* q,
                                    const double* k_x_bar, const double* k_x,
                                    const double* anchor_y, const double* anchor_kx, double* y_out,
                                    double* dy, double* k_out, double* k_dx) {
+  pdl_launch();
+  pdl_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
     const double yi = y[i];
@@ -355,7 +365,8 @@ int anu_backend_multiply(uint64_t id, const double* x, double* y) {
     auto it = s.matrices.find(id);
     if (it == s.matrices.end()) throw Error(ANU_ERR_INVALID, "matrix was not prepared");
     anu::Timed t(s, "multiply");
-    anu::product<double, double, double>(s.exec, *it->second, x, 1, anu::StoreEpi<double>{1, y});
+    anu::product<double, double, double>(s.exec, *it->second, x, 1, anu::StoreEpi<double>{1, y},
+                                         true);
   });
 }
 
@@ -392,9 +403,8 @@ int anu_backend_primal_update(int64_t n, double tau, double gamma, double halper
   return anu::guard([&](BackendState& s) {
     if (n <= 0) return;
     anu::Timed t(s, "primal update");
-    anu::primal_update_kernel<<<anu::grid_n(n), 256, 0, s.exec.stream>>>(
-        n, tau, gamma, halpern, x, c, kt_y, lower, upper, anchor, x_out, dx, x_bar);
-    ANU_CUDA(cudaGetLastError());
+    anu::launch_dependent(s.exec, anu::grid_n(n), 256, anu::primal_update_kernel, n, tau, gamma,
+                          halpern, x, c, kt_y, lower, upper, anchor, x_out, dx, x_bar);
   });
 }
 
@@ -406,10 +416,9 @@ int anu_backend_dual_update(int64_t m, int64_t num_equalities, double sigma, dou
   return anu::guard([&](BackendState& s) {
     if (m <= 0) return;
     anu::Timed t(s, "dual update");
-    anu::dual_update_kernel<<<anu::grid_n(m), 256, 0, s.exec.stream>>>(
-        m, num_equalities, sigma, gamma, halpern, y, q, k_x_bar, k_x, anchor_y, anchor_kx, y_out,
-        dy, k_out, k_dx);
-    ANU_CUDA(cudaGetLastError());
+    anu::launch_dependent(s.exec, anu::grid_n(m), 256, anu::dual_update_kernel, m, num_equalities,
+                          sigma, gamma, halpern, y, q, k_x_bar, k_x, anchor_y, anchor_kx, y_out,
+                          dy, k_out, k_dx);
   });
 }
 

@@ -517,10 +517,10 @@ __device__ __forceinline__ Acc block_sum(Acc v, Acc* scratch) {
 
 // One LP, one row block per CTA. Each thread first loads its share of the
 // block's indices and values into registers (kPerThread of each, all issued
-// before any is used), together with the epilogue's vectors for its row;
-// none of that depends on the previous launch, so under programmatic
-// dependent launch it overlaps the predecessor's tail. After the wait it
-// gathers x for all its nonzeros at once and stores the products in shared
+// before any is used), together with the epilogue's constants for its row;
+// none of that depends on earlier launches, so under programmatic dependent
+// launch it overlaps them. After the wait it gathers x for all its nonzeros
+// and loads the epilogue's state at once and stores the products in shared
 // memory. Rows of at most kSerialRow nonzeros are then summed by their own
 // thread, left to right from zero - the reference's order, so FP64 sums of
 // short rows match it bit for bit. Longer rows are listed in row order and
