@@ -206,12 +206,12 @@ typedef struct anu_pdhg_options {
    * size sums every row in the same order, so the choice changes timing
    * only, never a result. The result reports the pair and the trial time. */
   int32_t tile_threads;
-  /* A matrix small enough (up to 8,192 rows and columns, 16,384 in a packed
-   * batch, its slices and the
-   * copies of y and x_bar within a CTA's shared memory, for a single LP no row
-   * longer than 1,024 nonzeros) runs its iterations in cluster-resident
-   * launches: one thread-block cluster of 16 CTAs (8 where 16 does not fit)
-   * per case, as long as most of them are resident at once. 0 (default):
+  /* A matrix small enough runs its iterations in cluster-resident launches:
+   * one thread-block cluster of 16 CTAs (8 where 16 does not fit) per case, as
+   * long as most of the cases' clusters are resident at once. Small enough:
+   * up to 8,192 rows and columns (16,384 in a packed batch), the slices of
+   * both matrices and the copies of y and x_bar within a CTA's shared memory,
+   * and for a single LP no row longer than 1,024 nonzeros. 0 (default):
    * launches of at most 32 iterations, between which other streams' clusters
    * get their turn. 1: one launch per check period. Larger matrices, stacks of
    * more cases, and use_graphs = 0 take two launches per iteration. Rows are
