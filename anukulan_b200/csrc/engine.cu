@@ -9,8 +9,10 @@
 // polish, the Farkas infeasibility test, the time limit and the stop flag.
 // What changes is where the work runs: the iteration is two fused kernels
 // (K'y + primal step, K x_bar + dual step) launched as CUDA-graph chunks of
-// one check period, and every check is a handful of device reductions whose
-// results (18 doubles per case) are the only thing that crosses the bus.
+// one check period, or, for small matrices, a few dozen iterations inside one
+// launch of thread-block clusters (cluster.cuh); and every check is a handful
+// of device reductions whose results (18 doubles per case) are the only thing
+// that crosses the bus.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>

@@ -3,11 +3,11 @@
 //
 // Each LP keeps its own problem (scaled matrix and transpose on the device,
 // its own stream and memory pool) and runs the same fused single-LP path as
-// anu_pdhg_run: two kernels per iteration, CUDA-graph-captured between
-// termination checks. The batch is fed to W host workers from one queue,
-// largest LP first. A worker that finishes an LP (retires it) takes the next
-// one (admits it) at once, so up to W LPs' kernel streams overlap on the GPU
-// at any time. Small LPs fill only a few SMs each, and running many of them
+// anu_pdhg_run: cluster-resident launches for the smaller LPs, two kernels per
+// iteration, CUDA-graph-captured between termination checks, for the others.
+// The batch is fed to W host workers from one queue, largest LP first. A worker
+// that finishes an LP (retires it) takes the next one (admits it) at once, so
+// up to W LPs' kernel streams overlap on the GPU at any time. Small LPs fill only a few SMs each, and running many of them
 // side by side is what fills the device.
 //
 // W is chosen by a short autotuning pass at creation unless the caller
