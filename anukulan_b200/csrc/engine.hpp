@@ -242,6 +242,8 @@ struct Problem : Exec {
   // its single-LP checks run on one stream, without a second branch, and
   // launch directly for the first kConcurrentDirect checks of a solve.
   bool concurrent = false;
+  // One of more than kClusterWorkers solved at once: it takes no clusters.
+  bool crowded = false;
   // How stacks of so many cases run as cluster-resident chunks, once asked
   // (cluster_plan).
   std::map<std::pair<int, int>, ClusterPlan> cluster_plans;
@@ -296,6 +298,12 @@ constexpr int kSplitStack = 16;
 // the whole device then; one of a packed batch shares it and takes clusters up
 // to kClusterThreadsMax.
 constexpr int kClusterThreadsAlone = 512;
+// Packed batches of more workers than this take no clusters: more than the
+// device keeps resident queue for their SMs and hold up the large LPs' launches
+// (256 LPs of 500 to 50,000 rows on 32 workers: 31.7 LPs/s with clusters, 33.6
+// without; 16 LPs of 500 to 20,000 rows on 8 workers: 25.8 ms with, 30.2
+// without).
+constexpr int kClusterWorkers = 8;
 // Iterations per cluster-resident launch, unless options.cluster_chunks asks
 // for whole check periods: other streams' clusters wait for a launch to end,
 // so long check periods are cut, and the cut costs little because the next

@@ -82,11 +82,16 @@ int host_threads() {
   return h == 0 ? 4 : static_cast<int>(h);
 }
 
+void set_crowded(anu_pdhg_packed& h, int w) {
+  for (auto& p : h.problems) p->crowded = w > kClusterWorkers;
+}
+
 // Nonzero x iterations per second of `w` workers solving an even sample of
 // w LPs of the batch for a few check periods each (a second pass, timed,
 // after one that fills the sample LPs' memory pools: it measures how w
 // solves share the device, not how w first-time allocations contend).
 double sample_rate(anu_pdhg_packed& h, int w) {
+  set_crowded(h, w);
   const int n = static_cast<int>(h.problems.size());
   anu_pdhg_options o = h.options;
   o.max_iterations = 4 * o.termination_check_frequency;
@@ -227,6 +232,7 @@ int anu_pdhg_packed_create(int32_t num_lps, const anu_lp* lps, const anu_pdhg_op
       return h->problems[a]->k.nnz() > h->problems[b]->k.nnz();
     });
     h->workers = workers > 0 ? workers : anu::tune_workers(*h);
+    anu::set_crowded(*h, h->workers);
     if (options->tile_threads == 0) anu::tune_tile(*h, h->workers);
     *handle = h.release();
   });
