@@ -87,27 +87,20 @@ struct UnrollPrimal {
   // registers cost more than the latency (15.4 ms per 60-case, 300-step forward
   // and backward, 19.8 ms with two ahead).
   static constexpr int kPrefetch = 0;
-  __device__ __forceinline__ Pre prefetch(int32_t row, int32_t k) const {
+  __device__ __forceinline__ NoStep now(int32_t) const { return {}; }
+  __device__ __forceinline__ Pre prefetch(int32_t j, int32_t k, NoStep = {}) const {
     Pre r;
-    constants(row, k, r, {});
-    state(row, k, r, {});
-    return r;
-  }
-  __device__ __forceinline__ NoParams params(int32_t) const { return {}; }
-  __device__ __forceinline__ void constants(int32_t j, int32_t k, Pre& r, NoParams) const {
     const size_t e = static_cast<size_t>(j) * K + k;
     r.c = c[e];
     r.lo = lo[e];
     r.hi = hi[e];
     r.tau = static_cast<T>(tau[k]);
-  }
-  __device__ __forceinline__ void state(int32_t j, int32_t k, Pre& r, NoParams) const {
-    const size_t e = static_cast<size_t>(j) * K + k;
     r.x = x[e];
     if (!restart) r.anchor = anchor[e];
+    return r;
   }
   __device__ __forceinline__ void finish(int32_t j, int32_t k, T kty, const Pre& r,
-                                         NoParams = {}) const {
+                                         NoStep = {}) const {
     const size_t e = static_cast<size_t>(j) * K + k;
     const T xj = r.x;
     const T u = sub(xj, mul(r.tau, sub(r.c, kty)));
@@ -142,24 +135,18 @@ struct UnrollDual {
     T q, sigma, y, anchor;
   };
   static constexpr int kPrefetch = 0;
-  __device__ __forceinline__ Pre prefetch(int32_t row, int32_t k) const {
+  __device__ __forceinline__ NoStep now(int32_t) const { return {}; }
+  __device__ __forceinline__ Pre prefetch(int32_t i, int32_t k, NoStep = {}) const {
     Pre r;
-    constants(row, k, r, {});
-    state(row, k, r, {});
-    return r;
-  }
-  __device__ __forceinline__ NoParams params(int32_t) const { return {}; }
-  __device__ __forceinline__ void constants(int32_t i, int32_t k, Pre& r, NoParams) const {
-    r.q = q[static_cast<size_t>(i) * K + k];
-    r.sigma = static_cast<T>(sigma[k]);
-  }
-  __device__ __forceinline__ void state(int32_t i, int32_t k, Pre& r, NoParams) const {
     const size_t e = static_cast<size_t>(i) * K + k;
+    r.q = q[e];
+    r.sigma = static_cast<T>(sigma[k]);
     r.y = y[e];
     if (!restart) r.anchor = anchor[e];
+    return r;
   }
   __device__ __forceinline__ void finish(int32_t i, int32_t k, T bar, const Pre& r,
-                                         NoParams = {}) const {
+                                         NoStep = {}) const {
     const size_t e = static_cast<size_t>(i) * K + k;
     const T yi = r.y;
     const T s = add(yi, mul(r.sigma, sub(r.q, bar)));
@@ -231,25 +218,19 @@ struct RevPrimal {
     uint8_t mask;
   };
   static constexpr int kPrefetch = 0;
-  __device__ __forceinline__ Pre prefetch(int32_t row, int32_t k) const {
+  __device__ __forceinline__ NoStep now(int32_t) const { return {}; }
+  __device__ __forceinline__ Pre prefetch(int32_t j, int32_t k, NoStep = {}) const {
     Pre r;
-    constants(row, k, r, {});
-    state(row, k, r, {});
-    return r;
-  }
-  __device__ __forceinline__ NoParams params(int32_t) const { return {}; }
-  __device__ __forceinline__ void constants(int32_t j, int32_t k, Pre& r, NoParams) const {
-    r.tau = tau[k];
-    r.mask = mask[static_cast<size_t>(j) * K + k];
-  }
-  __device__ __forceinline__ void state(int32_t j, int32_t k, Pre& r, NoParams) const {
     const size_t e = static_cast<size_t>(j) * K + k;
+    r.tau = tau[k];
+    r.mask = mask[e];
     r.x = xh[e];
     r.anchor = axh[e];
     r.grad = gc[e];
+    return r;
   }
   __device__ __forceinline__ void finish(int32_t j, int32_t k, T ktz, const Pre& r,
-                                         NoParams = {}) const {
+                                         NoStep = {}) const {
     const size_t e = static_cast<size_t>(j) * K + k;
     const T xplus = r.x;
     T m;
@@ -289,28 +270,22 @@ struct RevDual {
     uint8_t mask;
   };
   static constexpr int kPrefetch = 0;
-  __device__ __forceinline__ Pre prefetch(int32_t row, int32_t k) const {
+  __device__ __forceinline__ NoStep now(int32_t) const { return {}; }
+  __device__ __forceinline__ Pre prefetch(int32_t i, int32_t k, NoStep = {}) const {
     Pre r;
-    constants(row, k, r, {});
-    state(row, k, r, {});
-    return r;
-  }
-  __device__ __forceinline__ NoParams params(int32_t) const { return {}; }
-  __device__ __forceinline__ void constants(int32_t i, int32_t k, Pre& r, NoParams) const {
+    const size_t e = static_cast<size_t>(i) * K + k;
     r.tau = static_cast<T>(tau[k]);
     r.sigma = sigma[k];
-    if (mask_prev != nullptr) r.mask = mask_prev[static_cast<size_t>(i) * K + k];
-  }
-  __device__ __forceinline__ void state(int32_t i, int32_t k, Pre& r, NoParams) const {
-    const size_t e = static_cast<size_t>(i) * K + k;
+    if (mask_prev != nullptr) r.mask = mask_prev[e];
     r.y = yh[e];
     if (mask_prev != nullptr) {
       r.anchor = ayh[e];
       r.grad = gq[e];
     }
+    return r;
   }
   __device__ __forceinline__ void finish(int32_t i, int32_t k, T kuh, const Pre& r,
-                                         NoParams = {}) const {
+                                         NoStep = {}) const {
     const size_t e = static_cast<size_t>(i) * K + k;
     const T yt = add(r.y, mul(r.tau, kuh));
     if (mask_prev == nullptr) {

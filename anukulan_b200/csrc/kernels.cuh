@@ -81,22 +81,20 @@ template <class T> __device__ __forceinline__ T load(const T* p) { return __ldg(
 // predecessor, so all earlier launches are complete too. pdl_launch lets the
 // next launch start. Outside such a launch both are no-ops.
 //
-// The single-LP kernels (rows_kernel, ell_kernel) let their successor start at
-// once and wait only where they need the launch before. A kernel may therefore
-// run while the two launches before it still do: ahead of pdl_wait it reads
-// only what no kernel of the chunk writes (the matrix and its schedule, the
-// epilogue's constants(), the per-case parameters), and everything the chunk
-// writes - the gathered vector, the epilogue's state() - is read after it, with
-// plain loads: the read-only path is not kept coherent with kernels that
-// overlap. Against starting the successor after the wait, this takes its launch
-// and its index loads off the critical path: one iteration of a 60,007 x 90,010
-// LP in FP64 14.4 -> 12.4 us, of a 1,000 x 1,500 LP in FP32 3.95 -> 3.4 us.
+// The iteration kernels start their successor after their own wait, so when a
+// kernel starts everything two launches back is complete: ahead of the wait it
+// reads the matrix, the per-case parameters and its rows' own vectors, which
+// its predecessor does not write, and after it the gathered vector, which the
+// predecessor does.
 //
-// The case-stack kernel (seg_kernel) starts its successor after its wait
-// instead, so anything two launches back is complete when it starts and the
-// epilogue's vectors are read ahead too: its launches are long, and early
-// successors only take registers and issue slots from the running one (30
-// cases of the refinery stack: 8.3 us per iteration, 10.6 with early starts).
+// Starting the successor first of all overlaps more launches, but their CTAs
+// hold registers and issue slots while they only wait. It costs most where the
+// device is shared (256 packed LPs on 16 workers 31.8 LPs/s, after the wait
+// 34.0; 30 stacked cases 10.6 us per iteration, after the wait 8.3), and alone
+// it gains nothing over the form above (a 60,007 x 90,010 LP in FP64 12.9 us
+// per iteration and 12.0, a 200,000 x 300,000 one in FP32 25.0 and 24.5).
+// Kernels without such vectors (the backend's updates, the power iteration's)
+// do start it first: alone in their stream, all they can overlap is launches.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -161,20 +159,15 @@ enum : uint32_t {
 
 // ------------------------------------------------------------ epilogues
 //
-// An epilogue's inputs besides the product's sum: params(case) gives how the
-// case steps; constants(row, case, pre) loads what no kernel of a chunk
-// writes, state(row, case, pre) what earlier kernels of it wrote; finish()
-// takes the step.
+// An epilogue's inputs besides the product's sum: now(case) gives how the case
+// steps in this launch, prefetch() loads the row's own vectors, finish() takes
+// the step. The single-LP kernels read both ahead of the wait (read after the
+// sums instead, the parameters' latency shows: 15.6 us per iteration of a
+// 60,007 x 90,010 LP in FP64, ahead 13.3). seg_kernel holds several rows'
+// vectors per thread and has no registers left for it: its form of prefetch()
+// keeps the Halpern weight with them, its form of finish() reads the parameters
+// where they are used (two 30-case stacks: 10.5 us per iteration, ahead 11.0).
 
-struct NoParams {};
-
-// How one case steps in this launch.
-template <class T>
-struct StepNow {
-  T length;  // tau or sigma
-  double gamma, eta;
-  uint32_t mode;
-};
 enum : uint32_t {
   kStepActive = 1u,   // not retired
   kStepBlend = 2u,    // Halpern blend with the anchor
@@ -187,6 +180,16 @@ __device__ __forceinline__ uint32_t step_mode(const StepParams& p, int32_t it) {
   return kStepActive | (p.halpern ? (reset_now ? kStepAnchor : kStepBlend) : 0u) |
          (p.gamma != 0.0 ? kStepReflect : 0u);
 }
+
+// How one case steps in this launch.
+template <class T>
+struct StepNow {
+  T length;        // tau or sigma
+  T gamma, w, wc;  // reflection; the Halpern weight and its complement
+  uint32_t mode;
+};
+// An epilogue that takes no step.
+struct NoStep {};
 
 // The steps themselves, on one entry (backend.cpp:60-111).
 template <class T>
@@ -238,17 +241,11 @@ struct StoreEpi {
   Out* __restrict__ out;
   struct Pre {};
   static constexpr int kPrefetch = 2;  // the segment ranges alone
-  __device__ __forceinline__ NoParams params(int32_t) const { return {}; }
-  __device__ __forceinline__ Pre prefetch(int32_t, int32_t) const { return {}; }
-  __device__ __forceinline__ void constants(int32_t, int32_t, Pre&, NoParams) const {}
-  __device__ __forceinline__ void state(int32_t, int32_t, Pre&, NoParams) const {}
+  __device__ __forceinline__ NoStep now(int32_t) const { return {}; }
+  __device__ __forceinline__ Pre prefetch(int32_t, int32_t, NoStep = {}) const { return {}; }
   template <class Acc>
   __device__ __forceinline__ void finish(int32_t r, int32_t k, Acc s, const Pre&,
-                                         NoParams) const {
-    out[(size_t)r * K + k] = static_cast<Out>(s);
-  }
-  template <class Acc>
-  __device__ __forceinline__ void finish(int32_t r, int32_t k, Acc s, const Pre&) const {
+                                         NoStep = {}) const {
     out[(size_t)r * K + k] = static_cast<Out>(s);
   }
 };
@@ -277,30 +274,28 @@ struct PrimalEpi {
   static constexpr int kPrefetch = 2;  // items seg_kernel loads ahead per thread
   struct Pre {
     T c, lo, hi, x, anchor, sum;
-    double w;  // this iteration's Halpern weight (when blending)
+    double w;  // seg_kernel's: this iteration's Halpern weight (when blending)
   };
   // A retired case's lanes neither gather nor step.
   __device__ __forceinline__ bool live(int32_t k) const { return p[k].active != 0; }
-  __device__ __forceinline__ StepNow<T> params(int32_t k) const {
+  __device__ __forceinline__ StepNow<T> now(int32_t k) const {
     const StepParams& P = p[k];
-    return {static_cast<T>(P.tau), P.gamma, P.eta, step_mode(P, it)};
+    const uint32_t mode = step_mode(P, it);
+    const double w = (mode & kStepBlend) ? w_table[(size_t)it * K + k] : 1.0;
+    return {static_cast<T>(P.tau), static_cast<T>(P.gamma), static_cast<T>(w),
+            static_cast<T>(1.0 - w), mode};
   }
-  __device__ __forceinline__ void constants(int32_t j, int32_t k, Pre& r,
-                                            const StepNow<T>& now) const {
-    if (!(now.mode & kStepActive)) return;
+  __device__ __forceinline__ Pre prefetch(int32_t j, int32_t k, const StepNow<T>& s) const {
+    Pre r{};
+    if (!(s.mode & kStepActive)) return r;
     const size_t e = (size_t)j * K + k;
+    r.x = x_in[e];
     r.c = c[e];
     r.lo = lo[e];
     r.hi = hi[e];
-    r.w = (now.mode & kStepBlend) ? w_table[(size_t)it * K + k] : 1.0;
-  }
-  __device__ __forceinline__ void state(int32_t j, int32_t k, Pre& r,
-                                            const StepNow<T>& now) const {
-    if (!(now.mode & kStepActive)) return;
-    const size_t e = (size_t)j * K + k;
-    r.x = x_in[e];
-    r.anchor = (now.mode & kStepBlend) ? anchor[e] : static_cast<T>(0);
+    r.anchor = (s.mode & kStepBlend) ? anchor[e] : static_cast<T>(0);
     r.sum = (flags & kAccumulate) ? sum_x[e] : static_cast<T>(0);
+    return r;
   }
   __device__ __forceinline__ Pre prefetch(int32_t j, int32_t k) const {
     Pre r{};
@@ -317,48 +312,35 @@ struct PrimalEpi {
     r.sum = (flags & kAccumulate) ? sum_x[e] : static_cast<T>(0);
     return r;
   }
-  // Returns the new x_bar entry (0 for a retired case).
-  __device__ __forceinline__ T finish(int32_t j, int32_t k, T kty, const Pre& r,
-                                      const StepNow<T>& now) const {
-    if (!(now.mode & kStepActive)) return static_cast<T>(0);
+  // Writes the step; returns the new x_bar entry.
+  __device__ __forceinline__ T store(int32_t j, int32_t k, const PrimalMove<T>& o, T sum,
+                                     uint32_t mode) const {
     const size_t e = (size_t)j * K + k;
-    const PrimalMove<T> o =
-        primal_move<T>(r.x, r.c, r.lo, r.hi, r.anchor, kty, now.length,
-                       static_cast<T>(now.gamma),
-                       static_cast<T>(r.w), static_cast<T>(1.0 - r.w), now.mode);
     if (flags & kWriteDelta) dx[e] = o.d;
     x_bar[e] = o.x_bar;
     x_out[e] = o.next;
-    if (now.mode & kStepAnchor) anchor[e] = o.next;
-    if (flags & kAccumulate) sum_x[e] = add(r.sum, mul(static_cast<T>(now.eta), o.next));
+    if (mode & kStepAnchor) anchor[e] = o.next;
+    if (flags & kAccumulate) sum_x[e] = add(sum, mul(static_cast<T>(p[k].eta), o.next));
     return o.x_bar;
   }
-  // The same step for seg_kernel, which keeps several items' vectors at hand:
-  // it reads the parameters where they are used and so keeps fewer registers
-  // (an iteration of two 30-case stacks: 10.5 us, 11.0 through the form above).
+  // Returns the new x_bar entry (0 for a retired case).
+  __device__ __forceinline__ T finish(int32_t j, int32_t k, T kty, const Pre& r,
+                                      const StepNow<T>& s) const {
+    if (!(s.mode & kStepActive)) return static_cast<T>(0);
+    return store(j, k,
+                 primal_move<T>(r.x, r.c, r.lo, r.hi, r.anchor, kty, s.length, s.gamma, s.w, s.wc,
+                                s.mode),
+                 r.sum, s.mode);
+  }
   __device__ __forceinline__ T finish(int32_t j, int32_t k, T kty, const Pre& r) const {
     const StepParams& P = p[k];
-    if (!P.active) return static_cast<T>(0);
-    const size_t e = (size_t)j * K + k;
-    const T xj = r.x;
-    T v = sub(xj, mul(static_cast<T>(P.tau), sub(r.c, kty)));
-    if (v < r.lo) v = r.lo;
-    if (v > r.hi) v = r.hi;
-    const T d = sub(v, xj);
-    if (flags & kWriteDelta) dx[e] = d;
-    const T xb = add(v, d);
-    x_bar[e] = xb;
-    T next = v;
-    if (P.gamma != 0.0) next = add(next, mul(static_cast<T>(P.gamma), d));
-    const bool reset_now = P.reset_pending && it == 0;
-    if (P.halpern && !reset_now) {
-      const double w = r.w;
-      next = add(mul(static_cast<T>(w), next), mul(static_cast<T>(1.0 - w), r.anchor));
-    }
-    x_out[e] = next;
-    if (P.halpern && reset_now) anchor[e] = next;
-    if (flags & kAccumulate) sum_x[e] = add(r.sum, mul(static_cast<T>(P.eta), next));
-    return xb;
+    const uint32_t mode = step_mode(P, it);
+    if (!(mode & kStepActive)) return static_cast<T>(0);
+    return store(j, k,
+                 primal_move<T>(r.x, r.c, r.lo, r.hi, r.anchor, kty, static_cast<T>(P.tau),
+                                static_cast<T>(P.gamma), static_cast<T>(r.w),
+                                static_cast<T>(1.0 - r.w), mode),
+                 r.sum, mode);
   }
 };
 
@@ -391,31 +373,29 @@ struct DualEpi {
   static constexpr int kPrefetch = 2;
   struct Pre {
     T q, floor_v, y, kx, anchor_y, anchor_kx, sum;
-    double w;  // this iteration's Halpern weight (when blending)
+    double w;  // seg_kernel's: this iteration's Halpern weight (when blending)
   };
   // A retired case's lanes neither gather nor step.
   __device__ __forceinline__ bool live(int32_t k) const { return p[k].active != 0; }
-  __device__ __forceinline__ StepNow<T> params(int32_t k) const {
+  __device__ __forceinline__ StepNow<T> now(int32_t k) const {
     const StepParams& P = p[k];
-    return {static_cast<T>(P.sigma), P.gamma, P.eta, step_mode(P, it)};
+    const uint32_t mode = step_mode(P, it);
+    const double w = (mode & kStepBlend) ? w_table[(size_t)it * K + k] : 1.0;
+    return {static_cast<T>(P.sigma), static_cast<T>(P.gamma), static_cast<T>(w),
+            static_cast<T>(1.0 - w), mode};
   }
-  __device__ __forceinline__ void constants(int32_t i, int32_t k, Pre& r,
-                                            const StepNow<T>& now) const {
-    if (!(now.mode & kStepActive)) return;
-    const size_t e = (size_t)i * K + k;
-    r.q = q[e];
-    r.floor_v = (i >= num_eq && ylo) ? ylo[e] : static_cast<T>(0);
-    r.w = (now.mode & kStepBlend) ? w_table[(size_t)it * K + k] : 1.0;
-  }
-  __device__ __forceinline__ void state(int32_t i, int32_t k, Pre& r,
-                                            const StepNow<T>& now) const {
-    if (!(now.mode & kStepActive)) return;
+  __device__ __forceinline__ Pre prefetch(int32_t i, int32_t k, const StepNow<T>& s) const {
+    Pre r{};
+    if (!(s.mode & kStepActive)) return r;
     const size_t e = (size_t)i * K + k;
     r.y = y_in[e];
+    r.q = q[e];
     r.kx = kx_in[e];
-    r.anchor_y = (now.mode & kStepBlend) ? anchor_y[e] : static_cast<T>(0);
-    r.anchor_kx = (now.mode & kStepBlend) ? anchor_kx[e] : static_cast<T>(0);
+    r.floor_v = (i >= num_eq && ylo) ? ylo[e] : static_cast<T>(0);
+    r.anchor_y = (s.mode & kStepBlend) ? anchor_y[e] : static_cast<T>(0);
+    r.anchor_kx = (s.mode & kStepBlend) ? anchor_kx[e] : static_cast<T>(0);
     r.sum = (flags & kAccumulate) ? sum_y[e] : static_cast<T>(0);
+    return r;
   }
   __device__ __forceinline__ Pre prefetch(int32_t i, int32_t k) const {
     Pre r{};
@@ -433,67 +413,41 @@ struct DualEpi {
     r.sum = (flags & kAccumulate) ? sum_y[e] : static_cast<T>(0);
     return r;
   }
-  // Returns the new y entry (0 for a retired case).
-  __device__ __forceinline__ T finish(int32_t i, int32_t k, T bar, const Pre& r,
-                                      const StepNow<T>& now) const {
-    if (!(now.mode & kStepActive)) return static_cast<T>(0);
+  // Writes the step; returns the new y entry.
+  __device__ __forceinline__ T store(int32_t i, int32_t k, const DualMove<T>& o, T sum,
+                                     uint32_t mode) const {
     const size_t e = (size_t)i * K + k;
-    const DualMove<T> o = dual_move<T>(r.y, r.q, r.kx, i >= num_eq, r.floor_v, r.anchor_y,
-                                       r.anchor_kx, bar, now.length,
-                                       static_cast<T>(now.gamma),
-                                       static_cast<T>(r.w), static_cast<T>(1.0 - r.w), now.mode);
     if (flags & kWriteDelta) {
       dy[e] = o.d;
       if (k_dx) k_dx[e] = o.k_d;
     }
     y_out[e] = o.next_y;
     kx_out[e] = o.next_k;
-    if (now.mode & kStepAnchor) {
+    if (mode & kStepAnchor) {
       anchor_y[e] = o.next_y;
       anchor_kx[e] = o.next_k;
     }
-    if (flags & kAccumulate) sum_y[e] = add(r.sum, mul(static_cast<T>(now.eta), o.next_y));
+    if (flags & kAccumulate) sum_y[e] = add(sum, mul(static_cast<T>(p[k].eta), o.next_y));
     return o.next_y;
   }
-  // The same step for seg_kernel, which keeps several items' vectors at hand:
-  // it reads the parameters where they are used and so keeps fewer registers
-  // (an iteration of two 30-case stacks: 10.5 us, 11.0 through the form above).
+  // Returns the new y entry (0 for a retired case).
+  __device__ __forceinline__ T finish(int32_t i, int32_t k, T bar, const Pre& r,
+                                      const StepNow<T>& s) const {
+    if (!(s.mode & kStepActive)) return static_cast<T>(0);
+    return store(i, k,
+                 dual_move<T>(r.y, r.q, r.kx, i >= num_eq, r.floor_v, r.anchor_y, r.anchor_kx, bar,
+                              s.length, s.gamma, s.w, s.wc, s.mode),
+                 r.sum, s.mode);
+  }
   __device__ __forceinline__ T finish(int32_t i, int32_t k, T bar, const Pre& r) const {
     const StepParams& P = p[k];
-    if (!P.active) return static_cast<T>(0);
-    const size_t e = (size_t)i * K + k;
-    const T yi = r.y;
-    const T kx = r.kx;
-    T v = add(yi, mul(static_cast<T>(P.sigma), sub(r.q, bar)));
-    if (i >= num_eq && v < r.floor_v) v = r.floor_v;
-    const T d = sub(v, yi);
-    const T kd = mul(static_cast<T>(0.5), sub(bar, kx));
-    if (flags & kWriteDelta) {
-      dy[e] = d;
-      if (k_dx) k_dx[e] = kd;
-    }
-    T next_y = v;
-    T next_k = mul(static_cast<T>(0.5), add(bar, kx));
-    if (P.gamma != 0.0) {
-      next_y = add(next_y, mul(static_cast<T>(P.gamma), d));
-      next_k = add(next_k, mul(static_cast<T>(P.gamma), kd));
-    }
-    const bool reset_now = P.reset_pending && it == 0;
-    if (P.halpern && !reset_now) {
-      const double w = r.w;
-      const T wt = static_cast<T>(w);
-      const T wc = static_cast<T>(1.0 - w);
-      next_y = add(mul(wt, next_y), mul(wc, r.anchor_y));
-      next_k = add(mul(wt, next_k), mul(wc, r.anchor_kx));
-    }
-    y_out[e] = next_y;
-    kx_out[e] = next_k;
-    if (P.halpern && reset_now) {
-      anchor_y[e] = next_y;
-      anchor_kx[e] = next_k;
-    }
-    if (flags & kAccumulate) sum_y[e] = add(r.sum, mul(static_cast<T>(P.eta), next_y));
-    return next_y;
+    const uint32_t mode = step_mode(P, it);
+    if (!(mode & kStepActive)) return static_cast<T>(0);
+    return store(i, k,
+                 dual_move<T>(r.y, r.q, r.kx, i >= num_eq, r.floor_v, r.anchor_y, r.anchor_kx, bar,
+                              static_cast<T>(P.sigma), static_cast<T>(P.gamma),
+                              static_cast<T>(r.w), static_cast<T>(1.0 - r.w), mode),
+                 r.sum, mode);
   }
 };
 
@@ -517,11 +471,11 @@ __device__ __forceinline__ Acc block_sum(Acc v, Acc* scratch) {
 
 // One LP, one row block per CTA. Each thread first loads its share of the
 // block's indices and values into registers (kPerThread of each, all issued
-// before any is used), together with the epilogue's constants for its row;
-// none of that depends on earlier launches, so under programmatic dependent
-// launch it overlaps them. After the wait it gathers x for all its nonzeros
-// and loads the epilogue's state at once and stores the products in shared
-// memory. Rows of at most kSerialRow nonzeros are then summed by their own
+// before any is used), together with the epilogue's vectors for its row; none
+// of that is written by the launch before, so under programmatic dependent
+// launch it overlaps that one's tail. After the wait it gathers x for all its
+// nonzeros at once and stores the products in shared memory. Rows of at most
+// kSerialRow nonzeros are then summed by their own
 // thread, left to right from zero - the reference's order, so FP64 sums of
 // short rows match it bit for bit. Longer rows are listed in row order and
 // taken by whole warps (lane-strided partial sums, then a fixed shuffle
@@ -558,10 +512,27 @@ struct RowTile {
   static constexpr int kSlots = kNnz + kNnz / 32;
 };
 
+// CTAs of a step kernel (one with a PDHG step in its epilogue) per SM, which
+// says how many registers it may use. A step kernel holds a row's vectors and
+// eight gathers per thread; left alone, the compiler saves registers (40 in
+// FP32) by issuing the gathers in turn. FP32 takes 48 registers on ten CTAs of
+// 128 threads: a 120,001 x 180,002 random LP 15.8 -> 13.8 us per iteration, a
+// 200,000 x 300,000 power-law one 25.9 -> 24.5 (at eight CTAs, 64 registers,
+// 16.0 and 26.0). FP64, six of 128: a 60,007 x 90,010 power-law LP 12.0 us per
+// iteration, at 7, 8 and 9 CTAs 12.4, 12.8 and 13.9. The larger FP64 tile keeps
+// four (64 registers): it is the better one where more CTAs hide more of the
+// gathers' latency, as on the 200,000 x 300,000 LP relabelled (25.1 us, at
+// three CTAs 27.0). Other kernels are left to the compiler.
+template <class Acc, class Epi, int kThreads>
+constexpr int step_ctas() {
+  if (std::is_same_v<decltype(std::declval<const Epi&>().now(0)), NoStep>) return 1;
+  if (sizeof(Acc) == 4) return 10 * kRowThreads / kThreads;
+  return kThreads == kRowThreads ? 6 : 8 * kRowThreads / kThreads;
+}
+
 template <class V, class X, class Acc, class Epi, int kThreads = kRowThreads>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
     rows_kernel(CsrView<V> a, const X* x, Epi epi) {
-  pdl_launch();
   using Tile = RowTile<kThreads>;
   constexpr int kWarps = kThreads / 32;
   __shared__ Acc prod[Tile::kSlots];
@@ -579,10 +550,10 @@ __global__ void __launch_bounds__(kThreads)
     // One long row: strided partial sums over kLongWidth virtual lanes, then
     // a fixed-order tree over them.
     typename Epi::Pre pre{};
-    const auto now = epi.params(0);
-    if (t == 0) epi.constants(r0, 0, pre, now);
+    const auto now = epi.now(0);
+    if (t == 0) pre = epi.prefetch(r0, 0, now);
     pdl_wait();
-    if (t == 0) epi.state(r0, 0, pre, now);
+    pdl_launch();
     Acc s = 0;
     const int32_t end = nz0 + nnz;
     if (t < kLongWidth) {
@@ -625,20 +596,19 @@ __global__ void __launch_bounds__(kThreads)
   const bool has_row = t < nrows;
   int32_t rb = 0, re = 0;
   typename Epi::Pre pre{};
-  const auto now = epi.params(0);
+  const auto now = epi.now(0);
   if (has_row) {
     rb = a.start[r0 + t] - nz0;
     re = a.start[r0 + t + 1] - nz0;
-    epi.constants(r0 + t, 0, pre, now);
+    pre = epi.prefetch(r0 + t, 0, now);
   }
-  // ---- the gather reads the previous launch's output, the epilogue's state
-  // those of the launches before; all of these loads are in flight together
+  // ---- the gather reads the previous launch's output
   pdl_wait();
+  pdl_launch();
   Acc xv[kPerThread];
 #pragma unroll
   for (int q = 0; q < kPerThread; ++q)
     xv[q] = col[q] >= 0 ? static_cast<Acc>(x[col[q]]) : static_cast<Acc>(0);
-  if (has_row) epi.state(r0 + t, 0, pre, now);
 #pragma unroll
   for (int q = 0; q < kPerThread; ++q)
     if (col[q] >= 0) prod[prod_slot(q * kThreads + t)] = mul(static_cast<Acc>(val[q]), xv[q]);
@@ -737,26 +707,25 @@ __device__ __forceinline__ void load_ell_row(const int32_t* __restrict__ index,
 }
 
 template <class V, class X, class Acc, class Epi, int kThreads = kRowThreads>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
     ell_kernel(CsrView<V> a, const X* x, Epi epi) {
-  pdl_launch();
   const int32_t r = static_cast<int32_t>(blockIdx.x) * kThreads + static_cast<int32_t>(threadIdx.x);
   const bool has_row = r < a.rows;
   int32_t col[kEllWidth];
   V val[kEllWidth];
   typename Epi::Pre pre{};
-  const auto now = epi.params(0);
+  const auto now = epi.now(0);
   if (has_row) {
     load_ell_row(a.index, a.value, r, col, val);
-    epi.constants(r, 0, pre, now);
+    pre = epi.prefetch(r, 0, now);
   }
   // ---- the gathers read the previous launch's output
   pdl_wait();
+  pdl_launch();
   if (!has_row) return;
   Acc xv[kEllWidth];
 #pragma unroll
   for (int q = 0; q < kEllWidth; ++q) xv[q] = static_cast<Acc>(x[col[q]]);
-  epi.state(r, 0, pre, now);
   Acc s = 0;
 #pragma unroll
   for (int q = 0; q < kEllWidth; ++q)
@@ -1090,9 +1059,9 @@ __device__ __forceinline__ void chunk_phase(const CsrView<V>& a, const SegSlice<
 #pragma unroll
       for (int qq = 0; qq < kChunkPrefetch; ++qq)
         if (qq == q) r = pre[qq];
-      epi.finish(row, k, sum, r, epi.params(k));
+      epi.finish(row, k, sum, r);
     } else {
-      epi.finish(row, k, sum, epi.prefetch(row, k), epi.params(k));
+      epi.finish(row, k, sum, epi.prefetch(row, k));
     }
   }
 }

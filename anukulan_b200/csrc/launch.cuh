@@ -32,7 +32,7 @@ inline int grid_for(int64_t items, int per_block, int cap) {
 
 
 // Shared-memory carveout for rows_kernel. Its residency is set by registers:
-// in FP32 12 CTAs of 128 threads at 40 registers, which need about 75 KB of
+// in FP32 10 CTAs of 128 threads at 48 registers, which need about 63 KB of
 // shared memory, while the driver by default sizes the carveout for the
 // shared-memory limit alone (21 CTAs, 132 KB) and leaves the rest to L1. The
 // hint asks for what the register-bound CTAs need, so every CTA stays
