@@ -1225,7 +1225,7 @@ void run_polish(Problem& p, bool unit, const std::vector<const CaseData*>& paren
 template <class T>
 ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   ClusterPlan none;
-  if (p.m == 0 || p.n == 0 || p.dk.nnz == 0 || p.crowded) return none;
+  if (p.m == 0 || p.n == 0 || p.dk.nnz == 0) return none;
   // Before any schedule is built: the shares are even at best.
   const int most = p.concurrent ? kClusterThreadsMax : kClusterThreadsAlone;
   if (std::max(p.m, p.n) > 16 * most ||

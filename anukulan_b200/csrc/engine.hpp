@@ -242,8 +242,6 @@ struct Problem : Exec {
   // its single-LP checks run on one stream, without a second branch, and
   // launch directly for the first kConcurrentDirect checks of a solve.
   bool concurrent = false;
-  // One of more than kClusterWorkers solved at once: it takes no clusters.
-  bool crowded = false;
   // How stacks of so many cases run as cluster-resident chunks, once asked
   // (cluster_plan).
   std::map<std::pair<int, int>, ClusterPlan> cluster_plans;
@@ -296,14 +294,13 @@ constexpr int kSplitStack = 16;
 // The most threads per CTA, hence sixteenths of a matrix's rows and columns,
 // for a problem that has the device to itself. A larger matrix is quicker over
 // the whole device then; one of a packed batch shares it and takes clusters up
-// to kClusterThreadsMax.
+// to kClusterThreadsMax, whatever the number of workers: clusters beyond those
+// resident at once wait for SMs, but leave most of them to the others (256 LPs
+// of 500 to 50,000 rows, FP32, on 12 / 24 / 48 workers: 34.1, 34.0, 33.9 LPs/s
+// with clusters; 34.0, 33.4, 33.6 without; 32 LPs of 500 to 5,000 rows, 1,000
+// iterations, on 12 / 16 / 24: 26.4, 26.3, 26.9 ms with; 40.5, 40.0, - without;
+// in FP64 on 16: 26.2 with, 31.5 without).
 constexpr int kClusterThreadsAlone = 512;
-// Packed batches of more workers than this take no clusters: more than the
-// device keeps resident queue for their SMs and hold up the large LPs' launches
-// (256 LPs of 500 to 50,000 rows on 32 workers: 31.7 LPs/s with clusters, 33.6
-// without; 16 LPs of 500 to 20,000 rows on 8 workers: 25.8 ms with, 30.2
-// without).
-constexpr int kClusterWorkers = 8;
 // Iterations per cluster-resident launch, unless options.cluster_chunks asks
 // for whole check periods: other streams' clusters wait for a launch to end,
 // so long check periods are cut, and the cut costs little because the next

@@ -3,12 +3,13 @@
 //
 // Each LP keeps its own problem (scaled matrix and transpose on the device,
 // its own stream and memory pool) and runs the same fused single-LP path as
-// anu_pdhg_run: cluster-resident launches for the smaller LPs, two kernels per
-// iteration, CUDA-graph-captured between termination checks, for the others.
-// The batch is fed to W host workers from one queue, largest LP first. A worker
-// that finishes an LP (retires it) takes the next one (admits it) at once, so
-// up to W LPs' kernel streams overlap on the GPU at any time. Small LPs fill only a few SMs each, and running many of them
-// side by side is what fills the device.
+// anu_pdhg_run: cluster-resident launches for the smaller LPs, at any W, and two
+// kernels per iteration, CUDA-graph-captured between termination checks, for
+// the others. The batch is fed to W host workers from one queue, largest LP
+// first. A worker that finishes an LP (retires it) takes the next one (admits
+// it) at once, so up to W LPs' kernel streams overlap on the GPU at any time.
+// Small LPs fill only a few SMs each, and running many of them side by side is
+// what fills the device.
 //
 // W is chosen by a short autotuning pass at creation unless the caller
 // fixes it. Each candidate W runs W LPs, drawn evenly from the size order,
@@ -82,16 +83,11 @@ int host_threads() {
   return h == 0 ? 4 : static_cast<int>(h);
 }
 
-void set_crowded(anu_pdhg_packed& h, int w) {
-  for (auto& p : h.problems) p->crowded = w > kClusterWorkers;
-}
-
 // Nonzero x iterations per second of `w` workers solving an even sample of
 // w LPs of the batch for a few check periods each (a second pass, timed,
 // after one that fills the sample LPs' memory pools: it measures how w
 // solves share the device, not how w first-time allocations contend).
 double sample_rate(anu_pdhg_packed& h, int w) {
-  set_crowded(h, w);
   const int n = static_cast<int>(h.problems.size());
   anu_pdhg_options o = h.options;
   o.max_iterations = 4 * o.termination_check_frequency;
@@ -232,7 +228,6 @@ int anu_pdhg_packed_create(int32_t num_lps, const anu_lp* lps, const anu_pdhg_op
       return h->problems[a]->k.nnz() > h->problems[b]->k.nnz();
     });
     h->workers = workers > 0 ? workers : anu::tune_workers(*h);
-    anu::set_crowded(*h, h->workers);
     if (options->tile_threads == 0) anu::tune_tile(*h, h->workers);
     *handle = h.release();
   });

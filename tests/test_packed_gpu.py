@@ -47,6 +47,25 @@ def test_packed_fp32_autotuned_reaches_tolerance(engine, batch):
         assert abs(r.objective - objective) <= 1e-4 * max(1.0, abs(objective))
 
 
+@pytest.mark.parametrize("precision", [0, PRECISION_FP32])
+@pytest.mark.parametrize("workers", [4, 9])
+def test_packed_clusters_at_any_worker_count(engine, precision, workers):
+    """LPs that fit a cluster run cluster-resident launches however many workers
+    there are, and end where two plain launches per iteration do, bit for bit.
+    8,200 and 12,001 columns take 513 and 751 rows per CTA, more than a single
+    LP's cluster ever has."""
+    lps = [lpgen.sparse_random_lp(m, n, per, seed=5 + n)[0]
+           for m, n, per in [(100, 150, 8), (700, 1000, 8), (1000, 1500, 8), (1301, 2001, 6),
+                             (2000, 2500, 5), (900, 3000, 6), (333, 4001, 4), (2700, 4100, 4),
+                             (2500, 8200, 4), (2500, 12_001, 3)]]
+    kw = dict(max_iterations=81, polish_on_exit=0, polish_feasibility=0, precision=precision)
+    for lp, r in zip(lps, engine.solve_packed(lps, workers=workers, **kw)):
+        plain = engine.solve_pdhg(lp, use_graphs=0, **kw)
+        assert r.iterations == plain.iterations == 81
+        assert np.array_equal(r.x, plain.x) and np.array_equal(r.y, plain.y)
+        assert r.kernel_launches < 2 * 81 < plain.kernel_launches
+
+
 def test_packed_rejects_bad_input(engine, batch):
     lp, _ = batch[0]
     with pytest.raises(engine.EngineError):
