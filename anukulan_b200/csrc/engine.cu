@@ -1225,7 +1225,10 @@ void run_polish(Problem& p, bool unit, const std::vector<const CaseData*>& paren
 template <class T>
 ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   ClusterPlan none;
-  if (p.m == 0 || p.n == 0 || p.dk.nnz == 0) return none;
+  if (p.m == 0 || p.n == 0 || p.dk.nnz == 0 || max_len < kClusterLenMin) return none;
+  if (K == 1 && sizeof(T) == 8 && !p.concurrent &&
+      (std::max(p.m, p.n) > 16 * kClusterRowsFp64 || p.dk.nnz > 16 * kClusterNnzFp64))
+    return none;
   // Before any schedule is built: the shares are even at best.
   const int most = p.concurrent ? kClusterThreadsMax : kClusterThreadsAlone;
   if (std::max(p.m, p.n) > 16 * most ||

@@ -293,7 +293,10 @@ constexpr int kSplitStack = 16;
 
 // The most threads per CTA, hence sixteenths of a matrix's rows and columns,
 // for a problem that has the device to itself. A larger matrix is quicker over
-// the whole device then; one of a packed batch shares it and takes clusters up
+// the whole device then (us per iteration in FP32, clusters of more threads
+// against launches: 9,000 columns 4.2 and 3.9, 12,000 columns 5.0 and 4.0,
+// a refinery plan of 52 periods 5.3 and 4.3; at 8,190 columns 3.8 and 3.9); one
+// of a packed batch shares it and takes clusters up
 // to kClusterThreadsMax, whatever the number of workers: clusters beyond those
 // resident at once wait for SMs, but leave most of them to the others (256 LPs
 // of 500 to 50,000 rows, FP32, on 12 / 24 / 48 workers: 34.1, 34.0, 33.9 LPs/s
@@ -301,6 +304,22 @@ constexpr int kSplitStack = 16;
 // iterations, on 12 / 16 / 24: 26.4, 26.3, 26.9 ms with; 40.5, 40.0, - without;
 // in FP64 on 16: 26.2 with, 31.5 without).
 constexpr int kClusterThreadsAlone = 512;
+// In FP64 a single LP that has the device to itself leaves the clusters earlier:
+// sixteen SMs' FP64 units bound the phase from about 256 rows or 1,750 nonzeros
+// per CTA on. Clusters against launches, ms per 1,200 iterations with checks:
+// 8 nonzeros per column, 2,200 rows 6.9 and 7.05, 2,600 rows 7.0 and 6.9, 4,000
+// rows 8.5 and 7.0; refinery plans of 14, 16 and 24 periods 7.1 and 7.3, 7.4 and
+// 7.3, 8.4 and 7.6; 6,000 columns of 4 nonzeros 8.0 and 6.8, 8,100 columns 9.8
+// and 7.0. (FP32 takes 8,100 columns in 7.5 and 7.9.) Stacks stay: their
+// launches are longer (3 cases of 24 periods 5.3 us per iteration and 18.2).
+constexpr int kClusterRowsFp64 = 256;
+constexpr int kClusterNnzFp64 = 1750;
+// The fewest iterations per launch: below, loading the slices costs more than
+// the iterations save (a check every iteration, 1,000 rows, ms per 1,200
+// iterations: FP32 80.0 and 75.9 by launches, FP64 60.2 and 55.4; every second
+// one 41.2 and 41.4, 34.3 and 29.0; every fifth 19.0 and 19.6, 15.9 and 15.1;
+// every tenth 11.5 and 12.9, 10.6 and 10.4).
+constexpr int kClusterLenMin = 5;
 // Iterations per cluster-resident launch, unless options.cluster_chunks asks
 // for whole check periods: other streams' clusters wait for a launch to end,
 // so long check periods are cut, and the cut costs little because the next

@@ -54,6 +54,29 @@ def test_small_shapes(engine, precision, shape):
     assert same(cluster, plain)
 
 
+# rows, columns, nonzeros per column, check period, whether FP64 and FP32 take
+# clusters.
+ROUTES = [(1000, 1500, 8, 40, True, True), (2000, 4096, 4, 40, True, True),
+          (2000, 4100, 4, 40, False, True), (1700, 3500, 8, 40, True, True),
+          (1700, 3504, 8, 40, False, True), (4000, 8190, 4, 40, False, True),
+          (4000, 8200, 4, 40, False, False), (1000, 1500, 8, 5, True, True),
+          (1000, 1500, 8, 4, False, False)]
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("route", ROUTES)
+def test_single_lp_routes(engine, precision, route):
+    m, n, per_col, period, fp64, fp32 = route
+    lp, _ = lpgen.sparse_random_lp(m, n, per_col)
+    kw = dict(max_iterations=120, polish_on_exit=0, polish_feasibility=0, precision=precision,
+              termination_check_frequency=period)
+    r, plain = engine.solve_pdhg(lp, **kw), engine.solve_pdhg(lp, use_graphs=0, **kw)
+    assert same(r, plain)
+    # A cluster launch takes the place of at least kClusterLenMin iterations.
+    saved = plain.kernel_launches - r.kernel_launches
+    assert saved >= 120 if (fp32 if precision else fp64) else saved < 20
+
+
 @pytest.mark.parametrize("precision", PRECISIONS)
 @pytest.mark.parametrize("cols", [8190, 8192, 8200])
 def test_largest_shapes(engine, precision, cols):
