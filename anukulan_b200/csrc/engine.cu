@@ -149,7 +149,6 @@ void DevCsr::prepare_cluster(const HostCsr& a, bool stack, int ctas, int32_t seg
   d.rows = {d.bounds.p, d.part_start.p, d.row.p, d.part.p, nullptr, d.entry.p,
             c.max_rows, c.max_entries, c.max_parts, c.stride};
   d.row_place = c.place;
-  d.max_row = c.max_row;
   d.ready = true;
 }
 
@@ -1212,16 +1211,24 @@ void run_polish(Problem& p, bool unit, const std::vector<const CaseData*>& paren
                                       states[which[w]].scales);
 }
 
-// How K cases on `p` run as cluster-resident chunks (cluster_chunk_kernel):
-// clusters of 16 CTAs (8 where the device takes no cluster of 16), one per
-// case. Not taken where a CTA's rows exceed its threads or its slices its
-// shared memory, where a single LP has a row longer than kLongRow (which more
-// than a warp sums), or where the stack needs more than four clusters for
-// every three that are resident at once: the others wait their turn, and a
-// stack of launches that each carry every case is quicker from there on (400
-// iterations of a 24-period refinery stack in FP32, 15 clusters resident, as
-// two half-stacks: 32 cases 10.8 ms against 12.3, 40 cases 13.1 against 13.5;
-// in FP64, 7 resident, one stack of 8: 6.1 against 7.8).
+// How K cases on `p` run as cluster-resident chunks (cluster_chunk_kernel): one
+// cluster of 16 or of 8 CTAs per case. Not taken where a CTA's rows exceed its
+// threads or its slices its shared memory, or where a single LP has a row
+// longer than kLongRow (which more than a warp sums). The size, by how many
+// clusters of it are resident at once (the others wait their turn):
+//  1. 16 CTAs, if every case's cluster is resident;
+//  2. 8 CTAs, if every case's cluster is: a case has half the SMs, but the cases
+//     run side by side (800 iterations, FP64, 8 cases of 16 periods 6.7 ms, two
+//     turns of clusters of 16 9.2, launches 9.4; 14 cases of it 7.1, launches
+//     9.7; 15 cases of 14 periods 6.8, 10.0 and 9.6; FP32, half-stacks of 15
+//     cases of 18 periods 9.9, 12.5 and 13.7);
+//  3. either, 16 before 8, up to four clusters for every three resident: from
+//     there on a stack of launches that each carry every case is quicker (24
+//     periods, FP64, 7 resident, 8 cases 10.9 ms against 13.3, 9 cases 11.0 and
+//     13.0; FP32, 15 resident, half-stacks of 16 cases 15.2 and 16.1, of 18 16.5
+//     and 16.3 to 17.9, of 20 17.0 to 18.4 and 17.6 to 18.7).
+// The count is that of this stack alone; where two half-stacks share the
+// device, their launches take turns, and the figures are for both together.
 template <class T>
 ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   ClusterPlan none;
@@ -1229,7 +1236,7 @@ ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   if (K == 1 && sizeof(T) == 8 && !p.concurrent &&
       (std::max(p.m, p.n) > 16 * kClusterRowsFp64 || p.dk.nnz > 16 * kClusterNnzFp64))
     return none;
-  // Before any schedule is built: the shares are even at best.
+  // The shares are even at best.
   const int most = p.concurrent ? kClusterThreadsMax : kClusterThreadsAlone;
   if (std::max(p.m, p.n) > 16 * most ||
       2 * sizeof(ClusterNz<T>) * (p.dk.nnz / 16) + sizeof(T) * (p.m + p.n) > kClusterSmemMax)
@@ -1237,27 +1244,50 @@ ClusterPlan cluster_plan(Problem& p, int K, int max_len) {
   const auto key = std::make_pair(K, max_len);
   const auto known = p.cluster_plans.find(key);
   if (known != p.cluster_plans.end()) return known->second;
-  ClusterPlan plan;
   const bool stack = K > 1;
-  for (const int ctas : {16, 8}) {
-    p.dk.prepare_cluster(p.k, stack, ctas, p.seg_nnz, p.stream);
-    p.dkt.prepare_cluster(p.kt, stack, ctas, p.seg_nnz, p.stream);
-    const DevCsr::Cluster &ck = p.dk.cluster(stack, ctas), &ckt = p.dkt.cluster(stack, ctas);
-    if (!stack && std::max(ck.max_row, ckt.max_row) > kLongRow) break;
-    const int32_t rows = std::max(ck.rows.max_rows, ckt.rows.max_rows);
-    if (rows > most) break;
+  // What one cluster size takes. `resident` is an upper bound (slices without
+  // padding) until the schedules are built, so that sizes which cannot serve
+  // build none.
+  struct Size {
+    int ctas, threads = 0, resident = 0;
+  } sizes[] = {{16}, {8}};
+  for (Size& s : sizes) {
+    const int32_t seg = stack ? p.seg_nnz : 0;
+    const ClusterShape k = cluster_shape(p.k, s.ctas, kSerialRow, seg, p.dk.seg_per_cta);
+    const ClusterShape kt = cluster_shape(p.kt, s.ctas, kSerialRow, seg, p.dkt.seg_per_cta);
+    const int32_t rows = std::max(k.max_rows, kt.max_rows);
+    if (rows > most || (!stack && std::max(k.max_row, kt.max_row) > kLongRow)) continue;
     // Threads for the rows, and as far as there is room for the sums apart
     // beside them: a warp each for a single LP, a thread each for a stack.
-    const int32_t parts = std::max(ck.rows.max_parts, ckt.rows.max_parts);
+    const int32_t parts = std::max(k.max_parts, kt.max_parts);
     const int32_t want = std::max(128, stack ? rows + parts : std::max(rows, 32 * parts));
-    const int threads = std::min((want + 31) / 32 * 32, std::max<int32_t>(kClusterThreadsAlone, (rows + 31) / 32 * 32));
-    const size_t smem = ClusterLayout::of<T>(ctas, ckt.rows, ck.rows, max_len).total;
-    const int resident = cluster_capacity<T>(cluster_kernel<T>(stack), ctas, threads, smem);
-    if (3 * K > 4 * resident) continue;
-    p.dk.place_cluster(p.k, ckt, stack, ctas, p.stream);
-    p.dkt.place_cluster(p.kt, ck, stack, ctas, p.stream);
-    plan = {ctas, threads, max_len};
-    break;
+    s.threads = std::min((want + 31) / 32 * 32,
+                         std::max<int32_t>(kClusterThreadsAlone, (rows + 31) / 32 * 32));
+    ClusterRows kr{}, ktr{};
+    for (auto [to, of] : {std::pair(&kr, &k), std::pair(&ktr, &kt)}) {
+      to->max_rows = of->max_rows;
+      to->max_entries = of->max_nnz;
+      to->max_parts = of->max_parts;
+      to->stride = (of->max_rows + 3) / 4 * 4;
+    }
+    s.resident = cluster_capacity<T>(cluster_kernel<T>(stack), s.ctas, s.threads,
+                                     ClusterLayout::of<T>(s.ctas, ktr, kr, max_len).total);
+  }
+  ClusterPlan plan;
+  for (const bool turns : {false, true}) {
+    for (Size& s : sizes) {
+      auto serves = [&]() { return turns ? 3 * K <= 4 * s.resident : K <= s.resident; };
+      if (plan.ctas != 0 || !serves()) continue;
+      p.dk.prepare_cluster(p.k, stack, s.ctas, p.seg_nnz, p.stream);
+      p.dkt.prepare_cluster(p.kt, stack, s.ctas, p.seg_nnz, p.stream);
+      const DevCsr::Cluster &ck = p.dk.cluster(stack, s.ctas), &ckt = p.dkt.cluster(stack, s.ctas);
+      s.resident = cluster_capacity<T>(cluster_kernel<T>(stack), s.ctas, s.threads,
+                                       ClusterLayout::of<T>(s.ctas, ckt.rows, ck.rows, max_len).total);
+      if (!serves()) continue;
+      p.dk.place_cluster(p.k, ckt, stack, s.ctas, p.stream);
+      p.dkt.place_cluster(p.kt, ck, stack, s.ctas, p.stream);
+      plan = {s.ctas, s.threads, max_len};
+    }
   }
   p.cluster_plans[key] = plan;
   return plan;

@@ -180,7 +180,6 @@ struct DevCsr {
     DevBuf<ClusterPart> part;
     ClusterRows rows{};
     std::vector<int32_t> row_place;
-    int32_t max_row = 0;
     bool ready = false;
   };
   Cluster clusters[2][2];

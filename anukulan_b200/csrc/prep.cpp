@@ -193,15 +193,39 @@ std::vector<RowBlock> row_blocks(const HostCsr& a, int32_t block_nnz, int32_t bl
   return blocks;
 }
 
+namespace {
+
+// Nonzeros per segment of a row of `len`: seg_nnz, or more where the row would
+// not fit a CTA's segments.
+int32_t segment_step(int32_t len, int32_t seg_nnz, int32_t seg_per_cta) {
+  return len > seg_nnz * seg_per_cta ? (len + seg_per_cta - 1) / seg_per_cta : seg_nnz;
+}
+
+// parts + 1 row bounds, cut where the running cost (a row's nonzeros plus
+// kClusterRowCost) crosses each part's even share.
+std::vector<int32_t> cluster_bounds(const HostCsr& a, int32_t parts) {
+  std::vector<int32_t> bounds(static_cast<size_t>(parts) + 1, a.rows);
+  bounds[0] = 0;
+  const int64_t total = a.nnz() + static_cast<int64_t>(kClusterRowCost) * a.rows;
+  int32_t part = 1;
+  for (int32_t r = 0; r < a.rows && part < parts; ++r) {
+    // Part `part` starts at the first row whose cost begins at or past its
+    // share; a row never splits.
+    const int64_t before = a.start[r] + static_cast<int64_t>(kClusterRowCost) * r;
+    while (part < parts && before * parts >= total * part) bounds[part++] = r;
+  }
+  return bounds;
+}
+
+}  // namespace
+
 SegmentSchedule segment_schedule(const HostCsr& a, int32_t seg_nnz, int32_t seg_per_cta,
                                  int32_t row_max) {
   SegmentSchedule s;
   s.row_seg.assign(static_cast<size_t>(a.rows) + 1, 0);
   for (int32_t r = 0; r < a.rows; ++r) {
     const int32_t b = a.start[r], e = a.start[r + 1];
-    const int32_t len = e - b;
-    int32_t step = seg_nnz;
-    if (len > seg_nnz * seg_per_cta) step = (len + seg_per_cta - 1) / seg_per_cta;
+    const int32_t step = segment_step(e - b, seg_nnz, seg_per_cta);
     s.row_seg[r] = static_cast<int32_t>(s.seg_begin.size());
     for (int32_t k = b; k < e; k += step) s.seg_begin.push_back(k);
   }
@@ -225,19 +249,33 @@ SegmentSchedule segment_schedule(const HostCsr& a, int32_t seg_nnz, int32_t seg_
   return s;
 }
 
+ClusterShape cluster_shape(const HostCsr& a, int32_t parts, int32_t serial_row, int32_t seg_nnz,
+                           int32_t seg_per_cta) {
+  ClusterShape s;
+  const std::vector<int32_t> bounds = cluster_bounds(a, parts);
+  for (int32_t q = 0; q < parts; ++q) {
+    int32_t apart = 0;
+    for (int32_t r = bounds[q]; r < bounds[q + 1]; ++r) {
+      const int32_t len = a.start[r + 1] - a.start[r];
+      s.max_row = std::max(s.max_row, len);
+      if (seg_nnz == 0) {
+        apart += len > serial_row ? 1 : 0;
+      } else {
+        const int32_t step = segment_step(len, seg_nnz, seg_per_cta);
+        if (len > step) apart += (len + step - 1) / step;
+      }
+    }
+    s.max_rows = std::max(s.max_rows, bounds[q + 1] - bounds[q]);
+    s.max_nnz = std::max(s.max_nnz, a.start[bounds[q + 1]] - a.start[bounds[q]]);
+    s.max_parts = std::max(s.max_parts, apart);
+  }
+  return s;
+}
+
 ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial_row,
                                  const SegmentSchedule* seg) {
   ClusterSchedule c;
-  c.bounds.assign(static_cast<size_t>(parts) + 1, a.rows);
-  c.bounds[0] = 0;
-  const int64_t total = a.nnz() + static_cast<int64_t>(kClusterRowCost) * a.rows;
-  int32_t part = 1;
-  for (int32_t r = 0; r < a.rows && part < parts; ++r) {
-    // Part `part` starts at the first row whose cost begins at or past its
-    // share; a row never splits.
-    const int64_t before = a.start[r] + static_cast<int64_t>(kClusterRowCost) * r;
-    while (part < parts && before * parts >= total * part) c.bounds[part++] = r;
-  }
+  c.bounds = cluster_bounds(a, parts);
   c.part_start.push_back(0);
   c.row.reserve(a.rows);
   c.entry.resize(a.index.size());
@@ -249,7 +287,6 @@ ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial
     // Here `first` is the sum's first nonzero; the layout below replaces it.
     for (int32_t r = rb; r < re; ++r) {
       const int32_t b = a.start[r], len = a.start[r + 1] - b;
-      c.max_row = std::max(c.max_row, len);
       const int32_t g0 = seg != nullptr ? seg->row_seg[r] : 0;
       const int32_t g1 = seg != nullptr ? seg->row_seg[r + 1] : (len > serial_row ? 2 : 1);
       if (g1 - g0 <= 1) {

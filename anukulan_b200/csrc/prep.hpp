@@ -114,10 +114,20 @@ struct ClusterSchedule {
   std::vector<int32_t> place;  // of each row: part * stride + its position in the part
   std::vector<int32_t> entry;  // of each nonzero, in its part's layout
   int32_t stride = 0;          // max_rows in whole 16-byte groups
-  int32_t max_row = 0;  // the longest row
   int32_t max_rows = 0, max_entries = 0, max_parts = 0;  // the most one part holds
 };
 constexpr int32_t kClusterRowCost = 4;
+
+// What the largest of `parts` parts of that schedule holds, without building it:
+// max_rows and max_parts are the schedule's, max_nnz its entries without the
+// layout's padding, max_row the longest row. seg_nnz and seg_per_cta are the segment
+// schedule's (segment_schedule) of a stack; seg_nnz 0: a single LP.
+struct ClusterShape {
+  int32_t max_row = 0, max_rows = 0, max_nnz = 0, max_parts = 0;
+};
+ClusterShape cluster_shape(const HostCsr& a, int32_t parts, int32_t serial_row, int32_t seg_nnz,
+                           int32_t seg_per_cta);
+
 ClusterSchedule cluster_schedule(const HostCsr& a, int32_t parts, int32_t serial_row,
                                  const SegmentSchedule* seg);
 

@@ -207,8 +207,9 @@ typedef struct anu_pdhg_options {
    * only, never a result. The result reports the pair and the trial time. */
   int32_t tile_threads;
   /* A matrix small enough runs its iterations in cluster-resident launches:
-   * one thread-block cluster of 16 CTAs (8 where 16 does not fit) per case, as
-   * long as most of the cases' clusters are resident at once. Small enough:
+   * one thread-block cluster per case, of 16 CTAs, or of 8 where only those are
+   * resident for every case at once, as long as at least three of four of the
+   * cases' clusters are. Small enough:
    * up to 8,192 rows and columns (16,384 in a packed batch), the slices of
    * both matrices and the copies of y and x_bar within a CTA's shared memory,
    * for a single LP no row longer than 1,024 nonzeros, and for a single LP in

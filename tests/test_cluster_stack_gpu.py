@@ -99,6 +99,30 @@ def test_stacks(engine, precision, cases):
         assert same(a, b)
 
 
+# Refinery periods, cases, precision, whether they take clusters. The device
+# keeps 7 clusters of 16 CTAs resident for FP64 plans of this size: 12 cases are
+# past four for every three of them, so they take clusters of 8; so do 8 cases,
+# which those serve at once. 24 periods leave no room for clusters of 8.
+STACK_ROUTES = [(16, 7, 0, True), (16, 8, 0, True), (16, 12, 0, True), (24, 8, 0, True),
+                (24, 10, 0, False), (18, 15, PRECISION_FP32, True),
+                (24, 15, PRECISION_FP32, True), (24, 24, PRECISION_FP32, False)]
+
+
+@pytest.mark.parametrize("route", STACK_ROUTES)
+def test_stack_routes(engine, route):
+    periods, cases, precision, clusters = route
+    stack = lpgen.refinery_stack(periods=periods)
+    sub = lpgen.CaseStack(stack.base, stack.names[:cases], stack.c[:cases], stack.q[:cases],
+                          stack.lower[:cases], stack.upper[:cases])
+    kw = dict(max_iterations=121, polish_on_exit=0, polish_feasibility=0, precision=precision,
+              split_stacks=0)
+    res = engine.solve_case_stack(sub, **kw)
+    plain = engine.solve_case_stack(sub, use_graphs=0, **kw)
+    assert all(same(a, b) for a, b in zip(res, plain))
+    saved = plain[0].kernel_launches - res[0].kernel_launches
+    assert saved >= 200 if clusters else saved < 20
+
+
 @pytest.mark.parametrize("precision", PRECISIONS)
 def test_rows_of_several_segments(engine, precision):
     stack = lpgen.long_row_stack(cases=5)  # three rows of 700 nonzeros
