@@ -8,6 +8,8 @@ equal exactly, in both precisions, on:
   rows and columns, and at and beyond what the CTAs' threads hold;
 - stacks of 2 cases up to more than the device keeps resident;
 - rows summed by warps (single LP) and in several segments (stack);
+- single LPs and stacks on both sides of every limit, with the route asserted
+  by the launches counted, stacks on clusters of 8 CTAs among them;
 - budgets that end inside a launch, and the averaged and KKT-restart schemes.
 """
 import numpy as np
@@ -52,6 +54,8 @@ def test_small_shapes(engine, precision, shape):
     cluster = engine.solve_pdhg(lp, **kw)
     plain = engine.solve_pdhg(lp, use_graphs=0, **kw)
     assert same(cluster, plain)
+    if precision or lp.k.nnz <= 28_000:
+        assert plain.kernel_launches - cluster.kernel_launches >= 140
 
 
 # rows, columns, nonzeros per column, check period, whether FP64 and FP32 take
@@ -94,9 +98,10 @@ def test_stacks(engine, precision, cases):
     sub = lpgen.CaseStack(stack.base, stack.names[pick], stack.c[pick], stack.q[pick],
                           stack.lower[pick], stack.upper[pick])
     kw = dict(max_iterations=95, polish_on_exit=0, polish_feasibility=0, precision=precision)
-    for a, b in zip(engine.solve_case_stack(sub, **kw),
-                    engine.solve_case_stack(sub, use_graphs=0, **kw)):
-        assert same(a, b)
+    res = engine.solve_case_stack(sub, **kw)
+    plain = engine.solve_case_stack(sub, use_graphs=0, **kw)
+    assert all(same(a, b) for a, b in zip(res, plain))
+    assert plain[0].kernel_launches - res[0].kernel_launches >= 150
 
 
 # Refinery periods, cases, precision, whether they take clusters. The device
@@ -127,9 +132,10 @@ def test_stack_routes(engine, route):
 def test_rows_of_several_segments(engine, precision):
     stack = lpgen.long_row_stack(cases=5)  # three rows of 700 nonzeros
     kw = dict(max_iterations=120, polish_on_exit=0, polish_feasibility=0, precision=precision)
-    for a, b in zip(engine.solve_case_stack(stack, **kw),
-                    engine.solve_case_stack(stack, use_graphs=0, **kw)):
-        assert same(a, b)
+    res = engine.solve_case_stack(stack, **kw)
+    plain = engine.solve_case_stack(stack, use_graphs=0, **kw)
+    assert all(same(a, b) for a, b in zip(res, plain))
+    assert plain[0].kernel_launches - res[0].kernel_launches >= 200
 
 
 @pytest.mark.parametrize("precision", PRECISIONS)

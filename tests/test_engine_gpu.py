@@ -338,8 +338,9 @@ def test_case_stack_tail_compaction(engine, stack):
 def test_case_stack_graphs_bit_identical(engine, stack, precision):
     # Iteration chunks, termination checks and re-centrings replayed as CUDA
     # graphs run the same kernels on the same buffers as direct launches:
-    # 20 cases (two half-stacks), results identical bit for bit.
-    sub = _rolling(stack, list(range(20)))
+    # 44 cases (two half-stacks, too many for clusters), results identical bit
+    # for bit.
+    sub = _rolling(stack, list(range(44)))
     kw = dict(tolerance=1e-6, precision=precision)
     graphs = engine.solve_case_stack(sub, use_graphs=1, **kw)
     direct = engine.solve_case_stack(sub, use_graphs=0, **kw)
@@ -348,6 +349,17 @@ def test_case_stack_graphs_bit_identical(engine, stack, precision):
         assert a.iterations == b.iterations and a.restarts == b.restarts, k
         assert np.array_equal(a.x, b.x) and np.array_equal(a.y, b.y), k
     assert graphs[0].refinement_rounds == direct[0].refinement_rounds
+
+
+@pytest.mark.parametrize("precision", [0, PRECISION_FP32])
+def test_single_lp_graphs_bit_identical(engine, precision):
+    # Too many columns for a cluster: iterations are graph-captured launches.
+    lp, _ = lpgen.sparse_random_lp(6000, 9000, 8)
+    kw = dict(max_iterations=250, polish_on_exit=0, polish_feasibility=0, precision=precision)
+    graphs, direct = engine.solve_pdhg(lp, **kw), engine.solve_pdhg(lp, use_graphs=0, **kw)
+    assert graphs.kernel_launches == direct.kernel_launches >= 500
+    assert graphs.iterations == direct.iterations and graphs.restarts == direct.restarts
+    assert np.array_equal(graphs.x, direct.x) and np.array_equal(graphs.y, direct.y)
 
 
 def _rolling(stack, idx):

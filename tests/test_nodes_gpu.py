@@ -1,6 +1,7 @@
 """Branch-and-bound node relaxations as one case stack
 (pdhg.solve_node_relaxations), against the engine's single solves, the
-reference's own solve_pdhg per node (oracle/_ref, cpu_backend) and HiGHS.
+reference's own solve_pdhg per node (oracle/_ref, cpu_backend; the oracle, which
+is pinned to it bit for bit, where that is not built) and HiGHS.
 
 The nodes are children of the refinery base case: the three columns whose
 root values are most fractional (among values >= 0.5), each branched down
@@ -45,10 +46,16 @@ def branch(lp, x, count):
     return np.array(lower), np.array(upper)
 
 
+def reference_solve(lp, **kw):
+    if oracle.have_reference():
+        return oracle.ref_solve(lp, threads=1, **kw)
+    return oracle.oracle_solve(lp, **kw)
+
+
 @pytest.fixture(scope="module")
 def nodes():
     lp = lpgen.refinery_stack().case(0)
-    root = oracle.ref_solve(lp, tolerance=1e-8)
+    root = reference_solve(lp, tolerance=1e-8)
     lower, upper = branch(lp, root.x, 3)
     lps = [lp.with_vectors(lower=lower[k], upper=upper[k]) for k in range(len(lower))]
     highs = [highs_objective(node) for node in lps]
@@ -77,7 +84,7 @@ def test_node_bounds_match_reference_and_highs(engine, nodes):
     stack = engine.solve_node_relaxations(lp, lower, upper, **KW)
     assert sum(nd.optimal for nd in stack) >= 3
     for k, nd in enumerate(stack):
-        ref = NodeRelaxation(oracle.ref_solve(lps[k], threads=1, **KW))
+        ref = NodeRelaxation(reference_solve(lps[k], **KW))
         assert nd.result.status == ref.result.status, k
         assert nd.optimal == ref.optimal, k
         status, optimum = highs[k]
