@@ -93,8 +93,12 @@ template <class T> __device__ __forceinline__ T load(const T* p) { return __ldg(
 // 34.0; 30 stacked cases 10.6 us per iteration, after the wait 8.3), and alone
 // it gains nothing over the form above (a 60,007 x 90,010 LP in FP64 12.9 us
 // per iteration and 12.0, a 200,000 x 300,000 one in FP32 25.0 and 24.5).
-// Kernels without such vectors (the backend's updates, the power iteration's)
-// do start it first: alone in their stream, all they can overlap is launches.
+// Kernels that read nothing of the kind ahead of their wait (a plain product, the
+// backend's updates, the power iteration's reduction and scaling) do start it
+// first: alone in their stream, all they can overlap is launches (a backend
+// iteration of a 1,000 x 1,500 LP 20.2 us with the products' successor after
+// their wait, 19.8 so; a check of 3,000 rows 47.9 and 47.5). A step kernel is
+// never launched as the dependent of one of these: a copy stands between.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -512,6 +516,10 @@ struct RowTile {
   static constexpr int kSlots = kNnz + kNnz / 32;
 };
 
+// A product that only stores its sums: no vectors of its own.
+template <class Epi>
+constexpr bool kPlain = std::is_empty_v<typename Epi::Pre>;
+
 // CTAs of a step kernel (one with a PDHG step in its epilogue) per SM, which
 // says how many registers it may use. A step kernel holds a row's vectors and
 // eight gathers per thread; left alone, the compiler saves registers (40 in
@@ -533,6 +541,7 @@ constexpr int step_ctas() {
 template <class V, class X, class Acc, class Epi, int kThreads = kRowThreads>
 __global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
     rows_kernel(CsrView<V> a, const X* x, Epi epi) {
+  if constexpr (kPlain<Epi>) pdl_launch();
   using Tile = RowTile<kThreads>;
   constexpr int kWarps = kThreads / 32;
   __shared__ Acc prod[Tile::kSlots];
@@ -553,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
     const auto now = epi.now(0);
     if (t == 0) pre = epi.prefetch(r0, 0, now);
     pdl_wait();
-    pdl_launch();
+    if constexpr (!kPlain<Epi>) pdl_launch();
     Acc s = 0;
     const int32_t end = nz0 + nnz;
     if (t < kLongWidth) {
@@ -604,7 +613,7 @@ __global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
   }
   // ---- the gather reads the previous launch's output
   pdl_wait();
-  pdl_launch();
+  if constexpr (!kPlain<Epi>) pdl_launch();
   Acc xv[kPerThread];
 #pragma unroll
   for (int q = 0; q < kPerThread; ++q)
@@ -709,6 +718,7 @@ __device__ __forceinline__ void load_ell_row(const int32_t* __restrict__ index,
 template <class V, class X, class Acc, class Epi, int kThreads = kRowThreads>
 __global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
     ell_kernel(CsrView<V> a, const X* x, Epi epi) {
+  if constexpr (kPlain<Epi>) pdl_launch();
   const int32_t r = static_cast<int32_t>(blockIdx.x) * kThreads + static_cast<int32_t>(threadIdx.x);
   const bool has_row = r < a.rows;
   int32_t col[kEllWidth];
@@ -721,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, step_ctas<Acc, Epi, kThreads>())
   }
   // ---- the gathers read the previous launch's output
   pdl_wait();
-  pdl_launch();
+  if constexpr (!kPlain<Epi>) pdl_launch();
   if (!has_row) return;
   Acc xv[kEllWidth];
 #pragma unroll
