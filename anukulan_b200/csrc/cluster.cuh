@@ -37,9 +37,9 @@
 // status, which the host reads; its CTA then goes straight to the
 // cluster barrier at the end, as its peers do when their own waits run out.
 //
-// Per iteration, against two launches per iteration: the 1,000 x 1,500 LP 2.3 us
-// (3.4) in FP32 and 3.2 (3.9) in FP64; a refinery plan of 24 periods 3.5 (4.5)
-// in FP32; 7 cases of it as a stack 3.2 (9.9) in FP32 and 5.3 (13.2) in FP64.
+// Per iteration, against two launches per iteration: a 1,000 x 1,500 LP 2.35 us
+// (3.7) in FP32 and 3.8 (4.0) in FP64; a refinery plan of 24 periods 3.3 (4.35)
+// in FP32; 12 cases of it as a stack 3.9 (8.2) in FP32, 7 in FP64 5.4 (13.0).
 //
 // The sums are the ones the two-launch path takes, in its order, so iterates
 // are the same bit for bit:
