@@ -294,14 +294,14 @@ constexpr int kSplitStack = 16;
 // for a problem that has the device to itself. A larger matrix is quicker over
 // the whole device then (us per iteration in FP32, clusters of more threads
 // against launches: 9,000 columns 4.2 and 3.9, 12,000 columns 5.0 and 4.0,
-// a refinery plan of 52 periods 5.3 and 4.3; at 8,190 columns 3.8 and 3.9); one
-// of a packed batch shares it and takes clusters up
-// to kClusterThreadsMax, whatever the number of workers: clusters beyond those
+// a refinery plan of 52 periods 5.3 and 4.3; at 8,190 columns 3.8 and 3.9).
+// One of a packed batch shares the device and takes clusters up to
+// kClusterThreadsMax, whatever the number of workers: clusters beyond those
 // resident at once wait for SMs, but leave most of them to the others (256 LPs
 // of 500 to 50,000 rows, FP32, on 12 / 24 / 48 workers: 34.1, 34.0, 33.9 LPs/s
-// with clusters; 34.0, 33.4, 33.6 without; 32 LPs of 500 to 5,000 rows, 1,000
-// iterations, on 12 / 16 / 24: 26.4, 26.3, 26.9 ms with; 40.5, 40.0, - without;
-// in FP64 on 16: 26.2 with, 31.5 without).
+// with clusters; 34.4, 33.4, 33.6 without; 32 LPs of 500 to 5,000 rows, 1,000
+// iterations, on 12 / 16: 26.4, 26.3 ms with; 40.5, 40.0 without; in FP64 on 16:
+// 26.2 with, 31.5 without).
 constexpr int kClusterThreadsAlone = 512;
 // In FP64 a single LP that has the device to itself leaves the clusters earlier:
 // sixteen SMs' FP64 units bound the phase from about 256 rows or 1,750 nonzeros

@@ -209,12 +209,11 @@ typedef struct anu_pdhg_options {
   /* A matrix small enough runs its iterations in cluster-resident launches:
    * one thread-block cluster per case, of 16 CTAs, or of 8 where only those are
    * resident for every case at once, as long as at least three of four of the
-   * cases' clusters are. Small enough:
-   * up to 8,192 rows and columns (16,384 in a packed batch), the slices of
-   * both matrices and the copies of y and x_bar within a CTA's shared memory,
-   * for a single LP no row longer than 1,024 nonzeros, and for a single LP in
-   * FP64 outside a packed batch up to 4,096 rows and columns and 28,000
-   * nonzeros. Check periods of fewer than 5 iterations take none. 0 (default):
+   * cases' clusters are. Small enough: up to 8,192 rows and columns (16,384 in
+   * a packed batch), the slices of both matrices and the copies of y and x_bar
+   * within a CTA's shared memory, for a single LP no row longer than 1,024
+   * nonzeros, and for a single LP in FP64 outside a packed batch up to 4,096
+   * rows and columns and 28,000 nonzeros. Check periods of fewer than 5 iterations take none. 0 (default):
    * launches of at most 32 iterations, between which other streams' clusters
    * get their turn. 1: one launch per check period. Larger matrices, stacks of
    * more cases, and use_graphs = 0 take two launches per iteration. Rows are
